@@ -408,6 +408,21 @@ static TuneKey tune_key(const chimera_handle* h) {
   return TuneKey(h->precision, h->riemann, h->limiter, h->mood, h->slope, cells, h->n);
 }
 
+// The tile variant of a new handle whose problem shape has not been autotuned.
+// FP64: variant 0, 32 x 16 tiles with TMA loads (rotor 1024^2 HLLE 520 us a
+// step, the next best 550).  FP32-bulk: variant 9, the same tile at three CTAs
+// an SM with TMA loads, the fastest for every solver (Kelvin-Helmholtz 4096^2
+// HLLD 4.84 ms a step against variant 0's 5.50, 2048^2 Rusanov 0.970 against
+// 1.134, rotor 1024^2 HLLE 280 us against 292).  FP32 on FP64 storage: variant
+// 1, three CTAs an SM (rotor 369 us against 382), but for HLLD, whose stage-2
+// and stage-3 fluxes that tile contracts differently in the last bit, variant 0.
+static int default_variant(const chimera_handle* h) {
+  if (h->variants.size() == 1) return 0;   // a mixed pair's one tile
+  if (h->precision == CHIMERA_FP32_BULK) return 9;
+  if (h->precision == CHIMERA_FP32_MIXED) return h->riemann == CHIMERA_RIEMANN_HLLD ? 0 : 1;
+  return 0;
+}
+
 extern "C" {
 
 int chimera_version(void) { return 10000; }
@@ -584,7 +599,7 @@ int chimera_batch_create(int n_members, const chimera_cfg* cfgs, void* stream, c
   }
   cudaMemcpyAsync(h->d_ctl, ctl.data(), sizeof(Control) * n_members, cudaMemcpyHostToDevice, h->stream);
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) { cudaGetLastError(); chimera_destroy(h); return CHIMERA_ERR_CUDA; }
-  int v0 = 0;
+  int v0 = default_variant(h);
   {
     std::lock_guard<std::mutex> lk(tune_mutex());
     auto it = tune_cache().find(tune_key(h));

@@ -5,8 +5,7 @@
 // L1, not bit for bit) spent on fewer instructions per cell:
 //   * phase 1.5 computes each cell's limited x and y slopes once into shared
 //     memory (the FP64 kernel recomputes them for each face that touches the
-//     cell, twice per direction), and the MOOD bounds either there too (SB)
-//     or in phase 2, once per low cell for its x and y faces;
+//     cell, twice per direction);
 //   * FP32 min / max / abs are the single hardware instructions;
 //   * the translation unit is compiled with fast FP32 division and square
 //     root (-use_fast_math), about 1 ulp instead of correctly rounded;
@@ -34,24 +33,22 @@
 
 namespace chimera {
 
-// Shared-memory plan.  SB: MOOD bounds stored per cell (12 arrays) or formed
-// in phase 2 from the primitives.  The new face-B arrays of phase 3a
-// reuse the slope arrays, which are dead once the face fluxes exist.
+// Shared-memory plan.  The new face-B arrays of phase 3a reuse the slope arrays,
+// which are dead once the face fluxes exist.
 // TMA staging: the six input fields over the box [i0-4, i0-4+BW) x [j0-3,
 // j0-3+BH) -- the primitives' 2-cell halo plus b_x(i-1), b_y(j-1) -- with the
 // box origin's x a multiple of 4 floats (16 bytes), each field's box padded to
 // 128 bytes, placed in the slope arrays after the face-B arrays.
-template <int TX, int TY, bool SB> struct TileGeom32 : TileGeom<TX, TY> {
+template <int TX, int TY> struct TileGeom32 : TileGeom<TX, TY> {
   using B = TileGeom<TX, TY>;
   static constexpr int SX = TX + 2, SY = TY + 2, NS = SX * SY;   // cells [i0-1, i0+TX] x [j0-1, j0+TY]
-  static constexpr int NSA = SB ? 24 : 12;                       // per-cell arrays: slopes (+ bounds)
   static_assert(B::NBX + B::NBY <= 12 * NS, "face-B arrays must fit in the slope arrays");
   static constexpr int BW = ((TX + 6 + 3) / 4) * 4, BH = TY + 5;  // TMA box (floats)
   static constexpr int BOXF = ((BW * BH + 31) / 32) * 32;        // one field's box, 128-byte multiple
   static constexpr int STG0 = ((B::NBX + B::NBY + 31) / 32) * 32; // staging offset in the slope arrays
   static constexpr bool TMA_FITS = STG0 + 32 + 6 * BOXF <= 12 * NS;   // (+32: 128-byte alignment slack)
   static constexpr size_t smem_bytes() {
-    return sizeof(float) * (size_t(6) * B::NP + size_t(NSA) * NS + size_t(5) * B::NFX + size_t(5) * B::NFY);
+    return sizeof(float) * (size_t(6) * B::NP + size_t(12) * NS + size_t(5) * B::NFX + size_t(5) * B::NFY);
   }
 };
 
@@ -62,6 +59,31 @@ template <int TX, int TY, bool SB> struct TileGeom32 : TileGeom<TX, TY> {
 template <int STAGE>
 __device__ __forceinline__ float rk_blend(float u0, float u) {
   return (STAGE == 2) ? u0 + 0.25f * (u - u0) : u0 + (2.0f / 3.0f) * (u - u0);
+}
+
+// The outflow boundary correction (src/main.f90:118-148) of a cell on the low
+// side with normal n: dt times the face length, a, times the physical flux of
+// the cell's own state (u, Bn normal, v, Bt tangential) added to mass, normal
+// and tangential momentum and energy.  Every rounding is spelled out: left to
+// the compiler, which of two products goes into a fused multiply-add varied
+// with the tile variant (one ulp in the momentum and energy of the boundary
+// cells).  hb2 is B^2 and w is v . B, the same values for both sides.  Stages 1
+// and 2 round the squares of B, stage 3 fuses them, as the first of this form's
+// tile variants always did.
+template <int STAGE>
+__device__ __forceinline__ void edge_inflow(float a, float gamma, float r, float u, float v, float P, float Bn,
+                                            float hb2, float w, float Bt, float& M, float& Mn, float& Mt, float& E) {
+  const float hb = __fmul_rn(0.5f, hb2);
+  const float vv = __fmaf_rn(v, v, __fmul_rn(u, u));
+  const float en = __fadd_rn(__fmaf_rn(__fmul_rn(0.5f, r), vv, __fdividef(__fsub_rn(P, hb), __fsub_rn(gamma, 1.0f))), hb);
+  const float ram = __fmaf_rn(r, __fmul_rn(u, u), P);
+  const float fn = (STAGE < 3) ? __fsub_rn(ram, __fmul_rn(Bn, Bn)) : __fmaf_rn(-Bn, Bn, ram);
+  const float ft = __fmaf_rn(__fmul_rn(r, u), v, -__fmul_rn(Bn, Bt));
+  const float fe = __fmaf_rn(__fadd_rn(en, P), u, -__fmul_rn(Bn, w));
+  M = __fmaf_rn(__fmul_rn(a, r), u, M);
+  Mn = __fmaf_rn(a, fn, Mn);
+  Mt = __fmaf_rn(a, ft, Mt);
+  E = __fmaf_rn(a, fe, E);
 }
 
 // A new face B of stage STAGE: b + dt * db (the curl of the FP32 corner Ez),
@@ -178,10 +200,10 @@ __device__ __forceinline__ void tma_issue(const StageArgs& a, int w, float* stg,
   for (int q = 0; q < 6; ++q) tma_load_2d(stg + q * BOXF, maps + q * TMAP_BYTES, i0 - 4, j0 - 3, bar);
 }
 
-template <int SOLVER, int STAGE, int TX, int TY, int NT, int MINB, bool SB, bool TMA, typename S = float,
+template <int SOLVER, int STAGE, int TX, int TY, int NT, int MINB, bool TMA, typename S = float,
           bool MIXBC = false>
 __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
-  using G = TileGeom32<TX, TY, SB>;
+  using G = TileGeom32<TX, TY>;
   static_assert(!TMA || G::TMA_FITS, "TMA staging must fit in the slope arrays");
   constexpr bool MIX = sizeof(S) == 8;   // FP64 storage, FP32 flux arithmetic
   static_assert(!(TMA && MIX), "the TMA staging holds FP32 boxes");
@@ -190,9 +212,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* sP = reinterpret_cast<R*>(smem_raw);       // [6][NP]   primitives, tile + 2 halo
   R* sS = sP + 6 * G::NP;                       // [12][NS]  slopes: field q, dir d at (2q+d)
-  R* sLo = sS + 12 * G::NS;                     // [6][NS]   MOOD lower bounds (SB)
-  R* sHi = sLo + 6 * G::NS;                     // [6][NS]   MOOD upper bounds (SB)
-  R* sFx = sS + G::NSA * G::NS;                 // [5][NFX]
+  R* sFx = sS + 12 * G::NS;                     // [5][NFX]
   R* sFy = sFx + 5 * G::NFX;                    // [5][NFY]
   S* sBx = reinterpret_cast<S*>(sS);            // new face B (phase 3a on): reuses the slopes
   S* sBy = sBx + G::NBX;
@@ -387,9 +407,9 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
     }
 
 
-    // ---- phase 1.5: per-cell slopes and MOOD bounds -----------------------------
+    // ---- phase 1.5: per-cell slopes ---------------------------------------------
     // apply_slope_limiter (src/mhd_derivatives.f90:50-127) or compute_gradients
-    // (:15-47); bounds of the 5-point stencil with the rho/P floor (:190-211).
+    // (:15-47).
     const R inv_dx = R(g.inv_dx), inv_dy = R(g.inv_dy);
     const R inv_2dx = R(g.inv_2dx), inv_2dy = R(g.inv_2dy);
     for (int c = tid; c < G::NS; c += NT) {
@@ -425,51 +445,17 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
         }
         sS[(2 * q + 0) * G::NS + c] = sx;
         sS[(2 * q + 1) * G::NS + c] = sy;
-        if (SB && mood_on) {
-          R lo = fminf(fminf(fminf(fminf(f0, xp), xm), yp), ym);
-          const R hi = fmaxf(fmaxf(fmaxf(fmaxf(f0, xp), xm), yp), ym);
-          if (q == 0 || q == 3) lo = fmaxf(R(0.1e-8), lo);
-          sLo[q * G::NS + c] = lo;
-          sHi[q * G::NS + c] = hi;
-        }
       }
     }
     __syncthreads();
 
     // ---- phase 2: face fluxes ------------------------------------------------------
     // One work item per low cell of the slope grid: its x face (i+1/2, j) and
-    // its y face (i, j+1/2), where the tile needs them, share the cell's MOOD
-    // bounds (the 5-point stencil of src/mhd_derivatives.f90:190-211), which
-    // are formed once (SB: loaded once).
+    // its y face (i, j+1/2), where the tile needs them.
     unsigned mood_resets = 0;
     for (int c = tid; c < G::NS; c += NT) {
       const int cx = c % G::SX, cy = c / G::SX;
       const int pa = (cy + 1) * G::PX + (cx + 1);             // the low cell in the primitive grid
-      R lo[6], hi[6];
-      if (mood_on) {
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-          if (SB) {
-            lo[q] = sLo[q * G::NS + c];
-            hi[q] = sHi[q * G::NS + c];
-          } else {
-            const R* s = sP + q * G::NP;
-            const R f0 = s[pa];
-            R xp = s[pa + 1], xm = s[pa - 1], yp = s[pa + G::PX], ym = s[pa - G::PX];
-            if constexpr (MIXBC) {
-              const int gx = i0 + cx - 1, gy = j0 + cy - 1;
-              if (px && !pxh && gx == -1) xp = f0;
-              if (!px && pxh && gx == nx) xm = f0;
-              if (py && !pyh && gy == -1) yp = f0;
-              if (!py && pyh && gy == ny) ym = f0;
-            }
-            R l = fminf(fminf(fminf(fminf(f0, xp), xm), yp), ym);
-            hi[q] = fmaxf(fmaxf(fmaxf(fmaxf(f0, xp), xm), yp), ym);
-            if (q == 0 || q == 3) l = fmaxf(R(0.1e-8), l);
-            lo[q] = l;
-          }
-        }
-      }
 #pragma unroll 1
       for (int d = 0; d < 2; ++d) {
         const bool ydir = d == 1;
@@ -479,7 +465,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
         const int pb = pa + (ydir ? G::PX : 1);
         const R hh = R(ydir ? g.hy : g.hx);
         R L[6], Rv[6];
-        bool reset = false;
+        unsigned outside = 0;   // bit q: a state of field q is not between the low and the high cell's values
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
           const R f0 = sP[q * G::NP + pa], fp = sP[q * G::NP + pb];
@@ -496,15 +482,46 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
             const int gl = ydir ? j0 + cy - 1 : i0 + cx - 1;
             if (gl == -1 && (ydir ? (py && !pyh) : (px && !pxh))) vR = f0;
           }
-          if (mood_on) {   // bounds of the LOW cell, reset to its value (src/mhd_derivatives.f90:213-216)
-            if (vL < lo[q] || vL > hi[q]) { vL = f0; reset = true; }
-            if (vR < lo[q] || vR > hi[q]) { vR = f0; reset = true; }
-          }
-          if (q == 0 || q == 3) {
-            vL = fmaxf(vL, R(1.0e-8));
-            vR = fmaxf(vR, R(1.0e-8));
-          }
+          // The low and the high cell are two of the five cells of the MOOD bounds
+          // below: states between their two values (with the rho / P floor on the
+          // lower one) are inside, whatever the other three hold.  Limited slopes
+          // put them there up to rounding (against bounds formed once for a low
+          // cell's two faces: Kelvin-Helmholtz 4096^2 4.84 ms a step for 5.33, Rusanov
+          // 2048^2 0.970 for 1.093, the TMA variant).  (A NaN is in neither test's way: the
+          // minima and maxima skip it, here as in the bounds.)
+          R vlo = fminf(f0, fp);
+          if (q == 0 || q == 3) vlo = fmaxf(R(0.1e-8), vlo);
+          if (!(fminf(vL, vR) >= vlo && fmaxf(vL, vR) <= fmaxf(f0, fp))) outside |= 1u << q;
           L[q] = vL; Rv[q] = vR;
+        }
+        bool reset = false;
+        if (mood_on && outside != 0) {
+          // bounds of the LOW cell (the 5-point stencil with the rho / P floor,
+          // src/mhd_derivatives.f90:190-211), reset to its value (:213-216)
+#pragma unroll
+          for (int q = 0; q < 6; ++q) {
+            if (!((outside >> q) & 1u)) continue;
+            const R* s = sP + q * G::NP;
+            const R f0 = s[pa];
+            R xp = s[pa + 1], xm = s[pa - 1], yp = s[pa + G::PX], ym = s[pa - G::PX];
+            if constexpr (MIXBC) {
+              const int gx = i0 + cx - 1, gy = j0 + cy - 1;
+              if (px && !pxh && gx == -1) xp = f0;
+              if (!px && pxh && gx == nx) xm = f0;
+              if (py && !pyh && gy == -1) yp = f0;
+              if (!py && pyh && gy == ny) ym = f0;
+            }
+            R lo = fminf(fminf(fminf(fminf(f0, xp), xm), yp), ym);
+            const R hi = fmaxf(fmaxf(fmaxf(fmaxf(f0, xp), xm), yp), ym);
+            if (q == 0 || q == 3) lo = fmaxf(R(0.1e-8), lo);
+            if (L[q] < lo || L[q] > hi) { L[q] = f0; reset = true; }
+            if (Rv[q] < lo || Rv[q] > hi) { Rv[q] = f0; reset = true; }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 6; q += 3) {   // face floors of rho and P (:223-227)
+          L[q] = fmaxf(L[q], R(1.0e-8));
+          Rv[q] = fmaxf(Rv[q], R(1.0e-8));
         }
         if (L[3] - R(0.5) * (L[4] * L[4] + L[5] * L[5]) < K<R>::P_floor) {
 #pragma unroll
@@ -732,21 +749,12 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
       const R cr = sP[0 * G::NP + pc], cu = sP[1 * G::NP + pc], cv = sP[2 * G::NP + pc];
       const R cP = sP[3 * G::NP + pc], cBx = sP[4 * G::NP + pc], cBy = sP[5 * G::NP + pc];
       floor_hits += conserved_floors<R>(U[0], U[1], U[2], U[3], cBx, cBy, gamma, vol) ? 1u : 0u;
-      if (!px && i == 0) {
-        const R hb = R(0.5) * (cBx * cBx + cBy * cBy);
-        const R en = ((cP - hb) / (gamma - R(1)) + R(0.5) * cr * (cu * cu + cv * cv)) + hb;
-        U[0] = U[0] + ax * cr * cu;
-        U[1] = U[1] + ax * ((cr * (cu * cu) + cP) - cBx * cBx);
-        U[2] = U[2] + ax * (cr * cu * cv - cBx * cBy);
-        U[3] = U[3] + ax * ((en + cP) * cu - cBx * (cBx * cu + cBy * cv));
-      }
-      if (!py && j == 0) {
-        const R hb = R(0.5) * (cBx * cBx + cBy * cBy);
-        const R en = ((cP - hb) / (gamma - R(1)) + R(0.5) * cr * (cu * cu + cv * cv)) + hb;
-        U[0] = U[0] + ay * cr * cv;
-        U[2] = U[2] + ay * ((cr * (cv * cv) + cP) - cBy * cBy);
-        U[1] = U[1] + ay * (cr * cv * cu - cBy * cBx);
-        U[3] = U[3] + ay * ((en + cP) * cv - cBy * (cBy * cv + cBx * cu));
+      if ((!px && i == 0) || (!py && j == 0)) {
+        const R hb2 = (STAGE < 3) ? __fadd_rn(__fmul_rn(cBx, cBx), __fmul_rn(cBy, cBy))
+                                  : __fmaf_rn(cBx, cBx, __fmul_rn(cBy, cBy));
+        const R w = __fmaf_rn(cBx, cu, __fmul_rn(cBy, cv));
+        if (!px && i == 0) edge_inflow<STAGE>(ax, gamma, cr, cu, cv, cP, cBx, hb2, w, cBy, U[0], U[1], U[2], U[3]);
+        if (!py && j == 0) edge_inflow<STAGE>(ay, gamma, cr, cv, cu, cP, cBy, hb2, w, cBx, U[0], U[2], U[1], U[3]);
       }
       if (STAGE >= 2) {   // rk_blend, fields in pairs: u0 + c (u - u0)
         const float c = (STAGE == 2) ? 0.25f : (2.0f / 3.0f);

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from chimera_b200 import problems as P
-from chimera_b200.config import BC_OUTFLOW, HLLD, HLLE, MC, RUSANOV, VAN_LEER
+from chimera_b200.config import BC_OUTFLOW, FP32_BULK, HLLD, HLLE, MC, RUSANOV, VAN_LEER
 from tests.gpu_util import require_gpu
 
 pytestmark = pytest.mark.gpu
@@ -66,3 +66,25 @@ def test_nan_cell_bitwise(G, oracle, cell, field):
         for x, y in zip(s.get_stage_buffer(1), ref):
             assert np.array_equal(x, y, equal_nan=True), v
     s.close()
+
+
+@pytest.mark.parametrize("solver,variants", [(RUSANOV, range(11)), (HLLE, range(11)), (HLLD, (5, 6, 9, 10))])
+def test_fp32_outflow_sides_same_bits_in_every_variant(G, solver, variants):
+    """FP32-bulk with outflow sides: the boundary flux correction rounds the
+    same in every tile variant (HLLD: in the two-way and three-way resident
+    tiles that share one contraction of the solver itself)."""
+    cfg, st = P.orszag_tang(96, riemann=solver)
+    cfg = cfg.replace(bc=(BC_OUTFLOW,) * 4, precision=FP32_BULK)
+    u0 = _rough(cfg, st, 9)
+    s = G.Solver(cfg)
+    outs = []
+    for v in variants:
+        s.set_variant(v)
+        s.set_state(u0)
+        s.set_time(0.0)
+        s.step(3)
+        outs.append(s.get_state())
+    s.close()
+    for o in outs[1:]:
+        for x, y in zip(o, outs[0]):
+            assert np.array_equal(x, y)
