@@ -393,6 +393,14 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
 #pragma unroll
           for (int q = 0; q < 6; ++q)
             tma_load_2d(const_cast<R*>(stg) + q * BX::BOXF, maps + q * TMAP_BYTES, i0 - 4, j0 - 3, &s_bar);
+          if (STAGE >= 2) {
+            // U^n of the tile, which phase 3 reads with plain loads, into L2
+            // meanwhile (rotor 1024^2 520 -> 509 us a step, Kelvin-Helmholtz
+            // 2048^2 3.06 -> 3.02 ms, Rusanov 2048^2 1.86 -> 1.80 ms)
+            const char* m0 = reinterpret_cast<const char*>(g.tmap) + size_t(sbuf) * 6 * TMAP_BYTES;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) tma_prefetch_2d(m0 + q * TMAP_BYTES, i0 - 4, j0 - 3);
+          }
         }
         const bool ok = mbar_wait(&s_bar, s_phase, TMA_POLLS);
         for (int p = tid; p < G::NP && ok; p += NT) {

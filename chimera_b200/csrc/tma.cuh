@@ -41,6 +41,14 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, 
       : "memory");
 }
 
+// The same box into L2 only: a hint, nothing waits for it.
+__device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(
+                   reinterpret_cast<uint64_t>(tmap)),
+               "r"(x), "r"(y)
+               : "memory");
+}
+
 // Wait for the phase with parity `parity` of `bar` to complete, giving up
 // after max_iter polls; returns whether it completed.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, unsigned max_iter) {
