@@ -241,12 +241,17 @@ static int launch_raw(chimera_handle* h, const KernelEntry& k, int grid, int w_b
   return CHIMERA_OK;
 }
 
-static int grid_for(chimera_handle* h, const KernelEntry& k) {
+// CTAs of kernel k that the device holds at once.
+static int resident_ctas(const chimera_handle* h, const KernelEntry& k) {
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.nt, k.smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   cudaGetLastError();
-  return std::max(1, std::min(h->total_tiles, per_sm * h->num_sms));
+  return per_sm * h->num_sms;
+}
+
+static int grid_for(chimera_handle* h, const KernelEntry& k) {
+  return std::max(1, std::min(h->total_tiles, resident_ctas(h, k)));
 }
 
 static int ensure_dt(chimera_handle* h) {
@@ -408,16 +413,37 @@ static TuneKey tune_key(const chimera_handle* h) {
   return TuneKey(h->precision, h->riemann, h->limiter, h->mood, h->slope, cells, h->n);
 }
 
+// The small-grid variants of a precision, smallest tile first.
+static std::vector<int> small_variants(const chimera_handle* h) {
+  if (h->variants.size() == 1) return {};   // a mixed pair's one tile
+  if (h->precision == CHIMERA_FP64) return {7, 8, 9};
+  if (h->precision == CHIMERA_FP32_MIXED) return {4, 5, 6};
+  // HLLD on the 8 x 8 tile contracts differently in the last bit: left out
+  if (h->riemann == CHIMERA_RIEMANN_HLLD) return {12, 13};
+  return {11, 12, 13};
+}
+
 // The tile variant of a new handle whose problem shape has not been autotuned.
-// FP64: variant 0, 32 x 16 tiles with TMA loads (rotor 1024^2 HLLE 520 us a
-// step, the next best 550).  FP32-bulk: variant 9, the same tile at three CTAs
+// Small grids: the first small-grid variant of which the device holds every
+// tile at once.  A tile's time is then a step's time, and it falls with the
+// faces a thread works through (Orszag-Tang FP64, us a step: 64^2 29 on 8 x 8
+// tiles, 39 on 16 x 8, 43 on 16 x 16, 66 on 32 x 16; 192^2 50, 42, 43, 68;
+// 256^2 85, 70, 52, 67, of which the device holds all 16 x 16 tiles but only
+// 296 of the 8 x 8 and 16 x 8 ones; rotor 320^2 125, 103, 83, 83).
+// Larger grids, FP64: variant 0, 32 x 16 tiles with TMA loads (rotor 1024^2
+// HLLE 509 us a step, the next best 550).  FP32-bulk: variant 9, the same tile at three CTAs
 // an SM with TMA loads, the fastest for every solver (Kelvin-Helmholtz 4096^2
 // HLLD 4.84 ms a step against variant 0's 5.50, 2048^2 Rusanov 0.970 against
 // 1.134, rotor 1024^2 HLLE 280 us against 292).  FP32 on FP64 storage: variant
 // 1, three CTAs an SM (rotor 369 us against 382), but for HLLD, whose stage-2
 // and stage-3 fluxes that tile contracts differently in the last bit, variant 0.
 static int default_variant(const chimera_handle* h) {
-  if (h->variants.size() == 1) return 0;   // a mixed pair's one tile
+  if (h->variants.size() == 1) return 0;
+  for (int v : small_variants(h)) {
+    const KernelEntry* k = h->variants[v].stage[h->riemann - 1];
+    const int tiles = tiles_for(h, k[0].tx, k[0].ty);
+    if (tiles <= std::min(resident_ctas(h, k[0]), std::min(resident_ctas(h, k[1]), resident_ctas(h, k[2])))) return v;
+  }
   if (h->precision == CHIMERA_FP32_BULK) return 9;
   if (h->precision == CHIMERA_FP32_MIXED) return h->riemann == CHIMERA_RIEMANN_HLLD ? 0 : 1;
   return 0;
@@ -1071,7 +1097,14 @@ int chimera_autotune(chimera_handle* h, int reps, int* chosen, double* best_ms) 
   h->profiling = 0;
   int best = h->cur_variant;
   float best_t = 1e30f;
+  const std::vector<int> small = small_variants(h);
   for (int v = 0; v < int(h->variants.size()) && rc == CHIMERA_OK; ++v) {
+    // no candidates: small-grid tiles the device would take in many waves (their
+    // halos make them slower there, by two at 2048^2)
+    const KernelEntry& k = h->variants[v].stage[h->riemann - 1][0];
+    if (std::find(small.begin(), small.end(), v) != small.end() &&
+        tiles_for(h, k.tx, k.ty) > 2 * resident_ctas(h, k))
+      continue;
     rc = layout(h, v);
     if (rc) break;
     h->dry = 1;

@@ -29,7 +29,7 @@ void fill(KernelSet* ks) {
 }  // namespace
 
 // Tile shapes and occupancy targets the autotuner chooses from.
-int fp32_variant_count() { return 11; }
+int fp32_variant_count() { return 14; }
 
 void fp32_kernels(int variant, KernelSet* out) {
   switch (variant) {
@@ -43,18 +43,25 @@ void fp32_kernels(int variant, KernelSet* out) {
     case 8: fill<64, 8, 256, 2>(out); break;
     case 9: fill<32, 16, 256, 3, true>(out); break;
     case 10: fill<16, 16, 128, 6, true>(out); break;
+    // small grids: fewer cells and faces a thread
+    case 11: fill<8, 8, 192, 2>(out); break;
+    case 12: fill<16, 8, 192, 3>(out); break;
+    case 13: fill<16, 16, 256, 3>(out); break;
     default: fill<32, 16, 256, 2>(out); break;
   }
 }
 
 // The FP32-arithmetic form on FP64 storage: the FP32-bulk tiles without TMA.
-int fp32m_variant_count() { return 4; }
+int fp32m_variant_count() { return 7; }
 
 void fp32m_kernels(int variant, KernelSet* out) {
   switch (variant) {
     case 1: fill<32, 16, 256, 3, false, double>(out); break;
     case 2: fill<32, 8, 128, 5, false, double>(out); break;
     case 3: fill<16, 16, 128, 6, false, double>(out); break;
+    case 4: fill<8, 8, 160, 3, false, double>(out); break;    // small grids
+    case 5: fill<16, 8, 192, 3, false, double>(out); break;
+    case 6: fill<16, 16, 256, 3, false, double>(out); break;
     default: fill<32, 16, 256, 2, false, double>(out); break;
   }
 }

@@ -27,7 +27,7 @@ void fill(KernelSet* ks) {
 
 // Tile shapes and occupancy targets the autotuner chooses from; the default
 // (variant 0) loads the stage input of interior tiles by TMA.
-int fp64_variant_count() { return 7; }
+int fp64_variant_count() { return 10; }
 
 void fp64_kernels(int variant, KernelSet* out) {
   switch (variant) {
@@ -37,6 +37,12 @@ void fp64_kernels(int variant, KernelSet* out) {
     case 4: fill<16, 16, 128, 4>(out); break;
     case 5: fill<32, 16, 256, 2, true>(out); break;   // phase 3b reads the stage input from shared memory
     case 6: fill<32, 16, 256, 1>(out); break;
+    // grids too small to give every SM two 32 x 16 tiles: a tile whose faces
+    // take the block one or two passes (180 faces on 192 threads, 332 on 192,
+    // 612 on 320) instead of five
+    case 7: fill<8, 8, 192, 2>(out); break;
+    case 8: fill<16, 8, 192, 2>(out); break;
+    case 9: fill<16, 16, 320, 2>(out); break;
     default: fill<32, 16, 256, 2, false, true>(out); break;   // phase 1 from TMA boxes (interior tiles)
   }
 }
