@@ -64,6 +64,15 @@ __device__ __forceinline__ int map_index(int g, int n, int plo, int phi) {
   return g < 0 ? 0 : n - 1;
 }
 
+// Programmatic dependent launch: the host lets a stage kernel start while the
+// one before it in the stream still runs.  grid_wait() holds until that one has
+// completed, its writes visible; everything a kernel reads comes after it.
+// grid_release(), once every CTA of a grid has called it or ended, lets the next
+// kernel's CTAs take up free places and wait there.  Both do nothing in an
+// ordinary launch.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <typename R> struct StageTileSmem;
 
 template <int TX, int TY> struct TileGeom {
@@ -343,6 +352,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
     }
     __syncthreads();
   }
+  grid_wait();
 
   for (int w = a.work_begin + blockIdx.x; w < a.total_tiles; w += gridDim.x) {
     const int m = (a.n_members == 1) ? 0 : a.tile_member[w];
@@ -608,6 +618,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
       unsigned s = __reduce_add_sync(0xffffffffu, mood_resets);
       if ((tid & 31) == 0 && s) atomicAdd(&ctl->mood_resets, (unsigned long long)s);
     }
+    if (w + int(gridDim.x) >= a.total_tiles) grid_release();   // the CTA's last tile: the next stage may take places
     __syncthreads();
 
     // the buffer pointers, read here rather than kept in registers through

@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
     return reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(sS + G::STG0) + 127) & ~uintptr_t(127));
   };
   constexpr unsigned TMA_POLLS = 1u << 26;   // bound of every wait for a TMA completion
+  grid_wait();
   if constexpr (TMA) {
     if (tid == 0) {
       mbar_init(&s_bar, 1);
@@ -554,6 +555,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
       unsigned s = __reduce_add_sync(0xffffffffu, mood_resets);
       if ((tid & 31) == 0 && s) atomicAdd(&ctl->mood_resets, (unsigned long long)s);
     }
+    if (w + int(gridDim.x) >= a.total_tiles) grid_release();   // the CTA's last tile: the next stage may take places
     __syncthreads();
     // the slopes are dead: the next tile's inputs stream in during phases 3a / 3b
     if constexpr (TMA) {

@@ -43,3 +43,37 @@ def test_large_grid_starts_on_the_large_tile(G, precision):
     cfg, _ = P.orszag_tang(512, riemann=HLLE)
     with G.Solver(cfg.replace(precision=precision)) as s:
         assert s.variant()["variant"] == LARGE[precision](HLLE)
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_BULK])
+@pytest.mark.parametrize("graph", [0, 2])
+def test_overlapped_launches_keep_stream_order(G, precision, graph):
+    """Stage kernels take places while the kernel before them finishes: two
+    handles of different tile shapes stepped in turn on one stream, with device
+    copies between, get what each gets alone."""
+    import torch
+    stream = torch.cuda.Stream()
+    grids = [P.orszag_tang(48, riemann=HLLE), P.rotor(320)]
+    alone, outs = [], []
+    for cfg, st in grids:
+        with G.Solver(cfg.replace(precision=precision)) as s:
+            s.set_state(st)
+            s.step(12)
+            alone.append(s.get_state())
+    pair = [G.Solver(cfg.replace(precision=precision), stream=stream.cuda_stream) for cfg, _ in grids]
+    for s, (_, st) in zip(pair, grids):
+        s.set_state(st)
+        s.set_graph_steps(graph)
+    dt = torch.empty(1, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(6):
+        for s in pair:
+            s.step(2)
+            s.get_dt_device(dt)
+            s.set_dt_device(dt)
+    outs = [s.get_state() for s in pair]
+    for s in pair:
+        s.close()
+    for a, b in zip(alone, outs):
+        for x, y in zip(a, b):
+            assert np.array_equal(x, y)
