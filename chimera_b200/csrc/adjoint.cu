@@ -4,29 +4,34 @@
 // lambda_n = (dU_{n+1}/dU_n)^T lambda_{n+1} with the time step held at its
 // forward value (the CFL dt is not differentiated: "frozen dt").
 //
-// Structure.  The step is re-run forward by simple per-cell / per-face "tape"
-// kernels that reproduce the fused stage kernel bit for bit (same device
-// functions, same operation order, --fmad=false) and record what the reverse
-// sweep needs: stage primitives, face fluxes, the pre-floor and pre-blend
-// conserved values, and per-face decision flags (MOOD resets, face floors,
-// thermal-pressure resets).  The reverse sweep then transposes, stage 3 to 1:
-//   floors + RK blend      (src/mhd_change_states.f90:116-166, src/main.f90:202-267)
-//   flux divergence        (src/mhd_flux.f90:20-76)
-//   constrained transport  (src/mhd_flux.f90:79-136): lambda_Ez at the corners
-//   Riemann solver         (src/mhd_flux.f90:197-779)
-//   thermal check, face floors, MOOD  (src/mhd_derivatives.f90:130-293): the
-//                          decisions are taken from the forward (a reset face
-//                          passes its adjoint to the cell it was reset to)
-//   slope limiter          (src/mhd_derivatives.f90:50-127); where a one-sided
-//                          difference is exactly zero (uniform neighbourhood) the
-//                          limiter is not differentiable: (1/2, 1/2) if both are
-//                          zero, else 1 w.r.t. the zero one (k_rev_slopes)
-//   primitive recovery     (src/mhd_change_states.f90:61-113)
-//   face->cell B average   (src/mhd_field_ops.f90:120-156)
-// as gather kernels (no atomics; deterministic).  Local Jacobians of the
-// pointwise functions come from evaluating the same templated device code
-// with forward-mode dual numbers (dual.cuh): at a kink (limiter branch, min /
-// max, floor) the derivative is that of the branch the forward took.
+// Structure.  The step is re-run forward by the fused FP64 stage kernels with the
+// tape (TapeOut): each stage leaves its primitives, a byte per cell that says
+// which floors changed the cell, and at those cells the values that went into
+// them.  The reverse sweep then transposes, stage 3 to 1, two kernels a stage:
+//   k_rev_faces  one thread a face: the adjoint of its five fluxes from the cells
+//                and corners around it --
+//                  floors + RK blend      (src/mhd_change_states.f90:116-166, src/main.f90:202-267)
+//                  flux divergence        (src/mhd_flux.f90:20-76)
+//                  constrained transport  (src/mhd_flux.f90:79-136): lambda_Ez at the corners
+//                -- the face states again from the primitives, with the forward's
+//                decisions, and the solver's vector-Jacobian product (face_vjp.cuh):
+//                  Riemann solver         (src/mhd_flux.f90:197-779)
+//                  thermal check, face floors, MOOD  (src/mhd_derivatives.f90:130-293): a
+//                                         reset face passes its adjoint to the cell it was reset to
+//   k_rev_cells  one thread a cell: gathers its faces' adjoints through
+//                  slope limiter          (src/mhd_derivatives.f90:50-127); where a one-sided
+//                                         difference is exactly zero (uniform neighbourhood) the
+//                                         limiter is not differentiable: (1/2, 1/2) if both are
+//                                         zero, else 1 w.r.t. the zero one (slope_vjp)
+//                  primitive recovery     (src/mhd_change_states.f90:61-113)
+//                  face->cell B average   (src/mhd_field_ops.f90:120-156)
+// as gathers (no atomics; deterministic).  At a kink (limiter branch, min / max,
+// floor) the derivative is that of the branch the forward took; the rarely taken
+// floors and the outflow correction are differentiated with forward-mode dual
+// numbers (dual.cuh) through the same device functions.
+//
+// This unit is compiled without multiply-add contraction: the face states repeat
+// the forward's bits and decisions.
 //
 // Boundary conditions: periodic or outflow (zero-gradient ghost cells), each
 // side on its own -- a periodic side may face an outflow one, whose faces and
@@ -40,11 +45,15 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 
 #include "../../include/chimera_gpu.h"
 #include "abi_check.h"
+#include "chimera_types.h"
 #include "dual.cuh"
+#include "face_vjp.cuh"
+#include "kernel_table.h"
 #include "mhd_device.cuh"
 
 using namespace chimera;
@@ -55,6 +64,7 @@ struct AdjGeom {
   int nx, ny;
   double dx, dy, inv_dx, inv_dy, inv_2dx, inv_2dy, hx, hy, gamma, vol;
   int riemann, limiter, slope, mood;
+  double igm1, ivol;   // 1 / (gamma - 1), 1 / vol
   int px, py;     // the low side (x = 0 / y = 0) is periodic (else outflow)
   int pxh, pyh;   // the high side is periodic (differs from the low side in a mixed pair)
 };
@@ -68,88 +78,25 @@ __device__ __forceinline__ int src(int i, int n, int plo, int phi) {
   return (i < 0 ? plo : phi) ? wrap(i, n) : (i < 0 ? 0 : n - 1);
 }
 
-// ---------------------------------------------------------------------------
-// forward tape kernels
-// ---------------------------------------------------------------------------
-struct StageTape {
-  double* P[6];      // stage primitives rho, vx, vy, P_total, Bx, By
-  double* Fx[5];     // x-face fluxes (face i+1/2): mass, momx, momy, energy, By
-  double* Fy[5];     // y-face fluxes (face j+1/2): mass, momx, momy, energy, Bx
-  uint32_t* flx;     // x-face decision flags
-  uint32_t* fly;     // y-face decision flags
-  double* Upre[4];   // conserved after the flux update, before the first floors
-  double* Ublend[4]; // conserved after the RK blend, before the second floors
+// One stage of the reverse sweep: what its two kernels read and write.
+struct RevStage {
+  AdjGeom g;
+  int stage;
+  double dt, c0, c1;               // RK blend weights of U^n and of the stage's update (0, 1 in stage 1)
+  const double* U[6];              // the stage's input
+  const double* lout[6];           // adjoint of the stage's output
+  TapeOut tape;
+  // per face (direction d: 0 x, 1 y; slot = the low cell) and field: the adjoints of
+  // the left and the right state that go on through the slopes, and, where the
+  // face's flag is set, what resets hand to the low cell's value directly
+  double* fL[2][6];
+  double* fR[2][6];
+  double* fX[2][6];
+  unsigned char* fflag[2];
+  double* lin[6];                  // adjoint of the stage's input
+  double* lU0[6];                  // adjoint of U^n through the blends: set in stage 3, added to in stage 2,
+                                   // added to lin in stage 1
 };
-
-__global__ void k_tape_prims(AdjGeom g, const double* const* __restrict__ U, StageTape t) {
-  const int n = g.nx * g.ny;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    const int i = c % g.nx, j = c / g.nx;
-    // average_face_to_cell_B: at an outflow low side the face value itself
-    const double Bx = (i > 0 || g.px) ? 0.5 * (U[4][c] + U[4][j * g.nx + wrap(i - 1, g.nx)]) : U[4][c];
-    const double By = (j > 0 || g.py) ? 0.5 * (U[5][c] + U[5][wrap(j - 1, g.ny) * g.nx + i]) : U[5][c];
-    Prim<double> p = get_primitive<double>(U[0][c], U[1][c], U[2][c], U[3][c], Bx, By, g.gamma, g.vol);
-    t.P[0][c] = p.rho; t.P[1][c] = p.vx; t.P[2][c] = p.vy;
-    t.P[3][c] = p.P; t.P[4][c] = p.Bx; t.P[5][c] = p.By;
-  }
-}
-
-// Face states of one face (low cell a, high cell b along direction d), with the
-// decision flags; the same operations as phase 2 of stage_kernel.
-template <typename R>
-__device__ __forceinline__ void face_states(const AdjGeom& g, const StageTape& t, int a, int b, int am, int bp,
-                                            int ax_p, int ax_m, int ay_p, int ay_m, bool ydir, bool b_own, R* L,
-                                            R* Rv, uint32_t* flags) {
-  const double inv_h = ydir ? g.inv_dy : g.inv_dx;
-  const double inv_2h = ydir ? g.inv_2dy : g.inv_2dx;
-  const double hh = ydir ? g.hy : g.hx;
-  uint32_t fl = 0;
-  for (int q = 0; q < 6; ++q) {
-    const double* s = t.P[q];
-    const double fm = s[am], f0 = s[a], fp = s[b], fpp = s[bp];
-    const double fb0 = b_own ? fp : f0;   // the high cell's low neighbour in its slope
-    double sa, sb;
-    if (g.slope) {
-      if (g.limiter == LIMITER_VAN_LEER) {
-        sa = limit_slope<double, LIMITER_VAN_LEER>((f0 - fm) * inv_h, (fp - f0) * inv_h);
-        sb = limit_slope<double, LIMITER_VAN_LEER>((fp - fb0) * inv_h, (fpp - fp) * inv_h);
-      } else {
-        sa = limit_slope<double, LIMITER_MC>((f0 - fm) * inv_h, (fp - f0) * inv_h);
-        sb = limit_slope<double, LIMITER_MC>((fp - fb0) * inv_h, (fpp - fp) * inv_h);
-      }
-    } else {
-      sa = (fp - fm) * inv_2h;
-      sb = (fpp - fb0) * inv_2h;
-    }
-    double vL = f0 + hh * sa;
-    double vR = fp - hh * sb;
-    const bool rp = (q == 0 || q == 3);
-    if (g.mood) {
-      double lo = dmin(dmin(dmin(dmin(f0, s[ax_p]), s[ax_m]), s[ay_p]), s[ay_m]);
-      const double hi = dmax(dmax(dmax(dmax(f0, s[ax_p]), s[ax_m]), s[ay_p]), s[ay_m]);
-      if (rp) lo = dmax(0.1e-8, lo);
-      if (vL < lo || vL > hi) { vL = f0; fl |= 1u << (4 * q + 0); }
-      if (vR < lo || vR > hi) { vR = f0; fl |= 1u << (4 * q + 1); }
-    }
-    if (rp) {
-      if (!(vL > 1.0e-8)) fl |= 1u << (4 * q + 2);
-      if (!(vR > 1.0e-8)) fl |= 1u << (4 * q + 3);
-      vL = dmax(vL, 1.0e-8);
-      vR = dmax(vR, 1.0e-8);
-    }
-    L[q] = R(vL);
-    Rv[q] = R(vR);
-  }
-  if (L[3] - R(0.5) * (L[4] * L[4] + L[5] * L[5]) < K<R>::P_floor) {
-    for (int q = 0; q < 6; ++q) L[q] = R(t.P[q][a]);
-    fl |= 1u << 24;
-  }
-  if (Rv[3] - R(0.5) * (Rv[4] * Rv[4] + Rv[5] * Rv[5]) < K<R>::P_floor) {
-    for (int q = 0; q < 6; ++q) Rv[q] = R(t.P[q][a]);
-    fl |= 1u << 25;
-  }
-  *flags = fl;
-}
 
 // neighbour indices for the face with low cell (i, j) in direction ydir
 struct FaceIdx {
@@ -186,43 +133,6 @@ __device__ __forceinline__ FaceIdx face_idx(const AdjGeom& g, int i, int j, bool
   return f;
 }
 
-template <int SOLVER>
-__global__ void k_tape_faces(AdjGeom g, StageTape t) {
-  const int n = g.nx * g.ny;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 2 * n; k += gridDim.x * blockDim.x) {
-    const bool ydir = k >= n;
-    const int c = ydir ? k - n : k;
-    const int i = c % g.nx, j = c / g.nx;
-    const FaceIdx f = face_idx(g, i, j, ydir);
-    double L[6], Rv[6];
-    uint32_t fl;
-    face_states<double>(g, t, f.a, f.b, f.am, f.bp, f.axp, f.axm, f.ayp, f.aym, ydir, f.b_own, L, Rv, &fl);
-    const double unL = ydir ? L[2] : L[1], unR = ydir ? Rv[2] : Rv[1];
-    const double utL = ydir ? L[1] : L[2], utR = ydir ? Rv[1] : Rv[2];
-    const double bnL = ydir ? L[5] : L[4], bnR = ydir ? Rv[5] : Rv[4];
-    const double btL = ydir ? L[4] : L[5], btR = ydir ? Rv[4] : Rv[5];
-    Flux5<double> F = riemann<double, SOLVER>(g.gamma, L[0], Rv[0], unL, unR, utL, utR, L[3], Rv[3], bnL, bnR, btL, btR);
-    double* const* dst = ydir ? t.Fy : t.Fx;
-    dst[0][c] = F.mass;
-    dst[1][c] = ydir ? F.momt : F.momn;
-    dst[2][c] = ydir ? F.momn : F.momt;
-    dst[3][c] = F.energy;
-    dst[4][c] = F.bt;
-    (ydir ? t.fly : t.flx)[c] = fl;
-  }
-}
-
-__device__ __forceinline__ double Ez_at(const AdjGeom& g, const StageTape& t, int i, int j) {
-  const int nx = g.nx, ny = g.ny;
-  i = wrap(i, nx);
-  j = wrap(j, ny);
-  const double fa = t.Fx[4][j * nx + i];
-  const double up = (j == ny - 1 && !g.pyh) ? fa : t.Fx[4][wrap(j + 1, ny) * nx + i];   // outflow: zero gradient
-  const double fb = t.Fy[4][j * nx + i];
-  const double right = (i == nx - 1 && !g.pxh) ? fb : t.Fy[4][j * nx + wrap(i + 1, nx)];
-  return 0.25 * (((-fa - up) + fb) + right);
-}
-
 // Outflow boundary flux correction (src/main.f90:118-148): a cell on an
 // outflow low side gets dt*dx times the physical flux of its own stage
 // primitives, in x (sx) and / or in y (sy).  Same operations as the fused
@@ -248,71 +158,6 @@ __device__ __forceinline__ void outflow_correction(bool sx, bool sy, R ax, R ay,
   }
 }
 
-__global__ void k_tape_update(AdjGeom g, int stage, double dt, const double* const* __restrict__ Uin,
-                              const double* const* __restrict__ U0, StageTape t, double* const* __restrict__ out) {
-  const int n = g.nx * g.ny;
-  const double ax = dt * g.dy, ay = dt * g.dx;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    const int i = c % g.nx, j = c / g.nx;
-    const int cxm = j * g.nx + wrap(i - 1, g.nx), cym = wrap(j - 1, g.ny) * g.nx + i;
-    double U[4];
-    for (int q = 0; q < 4; ++q) {
-      double F = Uin[q][c];
-      // at an outflow low side the incoming face flux is left out
-      if (i > 0 || g.px) F = (F - ax * t.Fx[q][c]) + ax * t.Fx[q][cxm];
-      else F = F - ax * t.Fx[q][c];
-      if (j > 0 || g.py) F = (F - ay * t.Fy[q][c]) + ay * t.Fy[q][cym];
-      else F = F - ay * t.Fy[q][c];
-      U[q] = F;
-      t.Upre[q][c] = F;
-    }
-    const double Bx = t.P[4][c], By = t.P[5][c];
-    conserved_floors<double>(U[0], U[1], U[2], U[3], Bx, By, g.gamma, g.vol);
-    outflow_correction<double>(!g.px && i == 0, !g.py && j == 0, ax, ay, g.gamma, t.P[0][c], t.P[1][c], t.P[2][c],
-                               t.P[3][c], Bx, By, U);
-    const double e0 = Ez_at(g, t, i, j);
-    // curl of -Ez; at an outflow low side the second row / column's difference
-    const double dbx = (j > 0 || g.py) ? ((-e0) - (-Ez_at(g, t, i, j - 1))) * g.inv_dy
-                                       : ((-Ez_at(g, t, i, 1)) - (-e0)) * g.inv_dy;
-    const double dby = (i > 0 || g.px) ? -(((-e0) - (-Ez_at(g, t, i - 1, j))) * g.inv_dx)
-                                       : -(((-Ez_at(g, t, 1, j)) - (-e0)) * g.inv_dx);
-    double bx = Uin[4][c] + dt * dbx;
-    double by = Uin[5][c] + dt * dby;
-    if (stage == 2) {
-      for (int q = 0; q < 4; ++q) U[q] = 0.75 * U0[q][c] + 0.25 * U[q];
-      bx = 0.75 * U0[4][c] + 0.25 * bx;
-      by = 0.75 * U0[5][c] + 0.25 * by;
-    } else if (stage == 3) {
-      for (int q = 0; q < 4; ++q) U[q] = (1.0 / 3.0) * U0[q][c] + (2.0 / 3.0) * U[q];
-      bx = (1.0 / 3.0) * U0[4][c] + (2.0 / 3.0) * bx;
-      by = (1.0 / 3.0) * U0[5][c] + (2.0 / 3.0) * by;
-    }
-    if (stage >= 2) {
-      for (int q = 0; q < 4; ++q) t.Ublend[q][c] = U[q];
-      conserved_floors<double>(U[0], U[1], U[2], U[3], Bx, By, g.gamma, g.vol);
-    }
-    for (int q = 0; q < 4; ++q) out[q][c] = U[q];
-    out[4][c] = bx;
-    out[5][c] = by;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// reverse kernels
-// ---------------------------------------------------------------------------
-struct RevBuf {
-  double* lUp[4];    // adjoint of the post-update (pre-floor) conserved values
-  double* lBc[2];    // adjoint of the stage cell B through the floors
-  double* lbp[2];    // adjoint of the post-CT face B
-  double* lEz;       // adjoint of the corner Ez
-  double* fX[24];    // x faces: per field q: lambda_fa, lambda_sa, lambda_fb, lambda_sb
-  double* fY[24];
-  double* w[24];     // per cell, field q, dir d: wL, wR at index (q*2+d)*2 + {0,1}
-  double* lPc[6];    // direct face adjoints to each cell's primitives
-  double* lB2[2];    // adjoint of cell Bx, By (for the face->cell average)
-  double* lPcor[6];  // adjoint of a cell's primitives through the outflow flux correction
-};
-
 // floors Jacobian-transpose product at inputs (M, Mx, My, E) with cell B
 __device__ __forceinline__ void floors_vjp(const AdjGeom& g, const double* Uin4, double Bx, double By,
                                            const double* lam4, double* out4, double* lB) {
@@ -329,62 +174,56 @@ __device__ __forceinline__ void floors_vjp(const AdjGeom& g, const double* Uin4,
   }
 }
 
-__global__ void k_rev_cells1(AdjGeom g, int stage, double stage_dt, const StageTape t,
-                             const double* const* __restrict__ lout, RevBuf r, double* const* __restrict__ lU0acc) {
-  const int n = g.nx * g.ny;
-  const double c0 = (stage == 2) ? 0.75 : (1.0 / 3.0);
-  const double c1 = (stage == 2) ? 0.25 : (2.0 / 3.0);
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    const double Bx = t.P[4][c], By = t.P[5][c];
-    double lB[2] = {0.0, 0.0};
-    double lpp[4];
-    double lbp0, lbp1;
-    if (stage >= 2) {
-      double ub[4] = {t.Ublend[0][c], t.Ublend[1][c], t.Ublend[2][c], t.Ublend[3][c]};
-      double lo[4] = {lout[0][c], lout[1][c], lout[2][c], lout[3][c]};
-      double lbl[4];
-      floors_vjp(g, ub, Bx, By, lo, lbl, lB);
-      for (int q = 0; q < 4; ++q) {
-        lU0acc[q][c] += c0 * lbl[q];
-        lpp[q] = c1 * lbl[q];
-      }
-      lU0acc[4][c] += c0 * lout[4][c];
-      lU0acc[5][c] += c0 * lout[5][c];
-      lbp0 = c1 * lout[4][c];
-      lbp1 = c1 * lout[5][c];
-    } else {
-      for (int q = 0; q < 4; ++q) lpp[q] = lout[q][c];
-      lbp0 = lout[4][c];
-      lbp1 = lout[5][c];
-    }
-    // outflow flux correction (added after the first floors): lpp is the
-    // adjoint of the correction too; through it to the cell's stage primitives
-    const int i = c % g.nx, j = c / g.nx;
-    const bool sx = !g.px && i == 0, sy = !g.py && j == 0;
-    double lcor[6] = {0, 0, 0, 0, 0, 0};
-    if (sx || sy) {
-      using D = Dual<6>;
-      const double ax = stage_dt * g.dy, ay = stage_dt * g.dx;
-      D pv[6];
-      for (int k = 0; k < 6; ++k) pv[k] = seed<6>(t.P[k][c], k);
-      D U[4] = {D(0.0), D(0.0), D(0.0), D(0.0)};
-      outflow_correction<D>(sx, sy, D(ax), D(ay), D(g.gamma), pv[0], pv[1], pv[2], pv[3], pv[4], pv[5], U);
-      for (int k = 0; k < 6; ++k) {
-        double sacc = 0.0;
-        for (int q = 0; q < 4; ++q) sacc += lpp[q] * U[q].d[k];
-        lcor[k] = sacc;
-      }
-    }
-    for (int k = 0; k < 6; ++k) r.lPcor[k][c] = lcor[k];
-    double up[4] = {t.Upre[0][c], t.Upre[1][c], t.Upre[2][c], t.Upre[3][c]};
-    double lu[4];
-    floors_vjp(g, up, Bx, By, lpp, lu, lB);
-    for (int q = 0; q < 4; ++q) r.lUp[q][c] = lu[q];
-    r.lBc[0][c] = lB[0];
-    r.lBc[1][c] = lB[1];
-    r.lbp[0][c] = lbp0;
-    r.lbp[1][c] = lbp1;
+// The adjoints at one cell whose floors changed it, or that carries the outflow
+// correction: lup (of the updated, pre-floor values), lbl (of the blend, before its
+// weights), lB (of the stage's cell B through the floors), lcor (of the stage's
+// primitives through the correction).  Rare: kept out of line.
+__device__ __noinline__ void cell_adjoint_slow(const RevStage& a, int c, double* lup, double* lbl, double* lB,
+                                               double* lcor) {
+  const unsigned hit = a.tape.hit[c];
+  const double Bx = a.tape.P[4][c], By = a.tape.P[5][c];
+  double l[4];
+  lB[0] = lB[1] = 0.0;
+  for (int q = 0; q < 4; ++q) l[q] = a.lout[q][c];
+  if (hit & 2u) {
+    const double ub[4] = {a.tape.Ublend[0][c], a.tape.Ublend[1][c], a.tape.Ublend[2][c], a.tape.Ublend[3][c]};
+    floors_vjp(a.g, ub, Bx, By, l, lbl, lB);
+  } else {
+    for (int q = 0; q < 4; ++q) lbl[q] = l[q];
   }
+  for (int q = 0; q < 4; ++q) l[q] = a.c1 * lbl[q];
+  const int i = c % a.g.nx, j = c / a.g.nx;
+  const bool sx = !a.g.px && i == 0, sy = !a.g.py && j == 0;
+  for (int k = 0; k < 6; ++k) lcor[k] = 0.0;
+  if (sx || sy) {   // added after the first floors: l is its adjoint too
+    using D = Dual<6>;
+    const double ax = a.dt * a.g.dy, ay = a.dt * a.g.dx;
+    D pv[6];
+    for (int k = 0; k < 6; ++k) pv[k] = seed<6>(a.tape.P[k][c], k);
+    D U[4] = {D(0.0), D(0.0), D(0.0), D(0.0)};
+    outflow_correction<D>(sx, sy, D(ax), D(ay), D(a.g.gamma), pv[0], pv[1], pv[2], pv[3], pv[4], pv[5], U);
+    for (int k = 0; k < 6; ++k)
+      for (int q = 0; q < 4; ++q) lcor[k] += l[q] * U[q].d[k];
+  }
+  if (hit & 1u) {
+    const double up[4] = {a.tape.Upre[0][c], a.tape.Upre[1][c], a.tape.Upre[2][c], a.tape.Upre[3][c]};
+    floors_vjp(a.g, up, Bx, By, l, lup, lB);
+  } else {
+    for (int q = 0; q < 4; ++q) lup[q] = l[q];
+  }
+}
+
+// The adjoint of a cell's updated, pre-floor conserved values.
+__device__ __forceinline__ void update_adjoint(const RevStage& a, int c, double* lup) {
+  if (a.tape.hit[c]) {
+    double lbl[4], lB[2], lcor[6], l[4];
+    cell_adjoint_slow(a, c, l, lbl, lB, lcor);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) lup[q] = l[q];
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) lup[q] = a.c1 * a.lout[q][c];
 }
 
 // lambda_Ez at corner (i+1/2, j+1/2): b_x(i,j) gets -dt/dy Ez(i,j), b_x(i,j+1)
@@ -392,247 +231,391 @@ __global__ void k_rev_cells1(AdjGeom g, int stage, double stage_dt, const StageT
 // At an outflow low side b_x(i,0) takes row 1's difference, dt/dy (Ez(i,0) -
 // Ez(i,1)), and b_y(0,j) column 1's, dt/dx (Ez(1,j) - Ez(0,j)); past an
 // outflow high side there is no b_x(i,ny) / b_y(nx,j).
-__global__ void k_rev_corners(AdjGeom g, double dt, RevBuf r) {
-  const int n = g.nx * g.ny;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    const int i = c % g.nx, j = c / g.nx;
-    const int cyp = wrap(j + 1, g.ny) * g.nx + i;
-    const int cxp = j * g.nx + wrap(i + 1, g.nx);
-    double sx = 0.0, sy = 0.0;
-    if (j + 1 < g.ny || g.py) sx += r.lbp[0][cyp];
-    if (j > 0 || g.py) sx -= r.lbp[0][c];
-    if (!g.py && j == 0) sx += r.lbp[0][i];
-    if (!g.py && j == 1) sx -= r.lbp[0][i];
-    if (i > 0 || g.px) sy += r.lbp[1][c];
-    if (i + 1 < g.nx || g.px) sy -= r.lbp[1][cxp];
-    if (!g.px && i == 0) sy -= r.lbp[1][j * g.nx];
-    if (!g.px && i == 1) sy += r.lbp[1][j * g.nx];
-    r.lEz[c] = dt * g.inv_dy * sx + dt * g.inv_dx * sy;
-  }
+__device__ __forceinline__ double corner_adjoint(const RevStage& a, int i, int j) {
+  const AdjGeom& g = a.g;
+  const double* lx = a.lout[4];
+  const double* ly = a.lout[5];
+  const int c = j * g.nx + i;
+  double sx = 0.0, sy = 0.0;
+  if (j + 1 < g.ny || g.py) sx += lx[wrap(j + 1, g.ny) * g.nx + i];
+  if (j > 0 || g.py) sx -= lx[c];
+  if (!g.py && j == 0) sx += lx[i];
+  if (!g.py && j == 1) sx -= lx[i];
+  if (i > 0 || g.px) sy += ly[c];
+  if (i + 1 < g.nx || g.px) sy -= ly[j * g.nx + wrap(i + 1, g.nx)];
+  if (!g.px && i == 0) sy -= ly[j * g.nx];
+  if (!g.px && i == 1) sy += ly[j * g.nx];
+  return a.c1 * (a.dt * g.inv_dy * sx + a.dt * g.inv_dx * sy);
 }
 
+// One face: blockIdx.y gives the direction.  Bound by latency, of the FP64 chains
+// of the slopes and the solver and of the loads before them, so by the warps in
+// flight: five blocks of 128 an SM at 96 registers (HLLD, which spills twice as
+// much there, four) ran a 512^2 HLLE launch in 61 us, four in 69, two at 214 in 118;
+// with twelve forward tangents instead of the transposed solver it took 136.
 template <int SOLVER>
-__global__ void k_rev_faces(AdjGeom g, double dt, StageTape t, RevBuf r) {
-  const int n = g.nx * g.ny;
-  const double ax = dt * g.dy, ay = dt * g.dx;
-  using D = Dual<12>;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 2 * n; k += gridDim.x * blockDim.x) {
-    const bool ydir = k >= n;
-    const int c = ydir ? k - n : k;
-    const int i = c % g.nx, j = c / g.nx;
-    const FaceIdx f = face_idx(g, i, j, ydir);
-    // adjoint of this face's 5 fluxes (conserved ordering)
+__global__ void __launch_bounds__(128, SOLVER == RIEMANN_HLLD ? 4 : 5) k_rev_faces(const __grid_constant__ RevStage a) {
+  const AdjGeom& g = a.g;
+  const bool ydir = blockIdx.y != 0;
+  const int d = ydir ? 1 : 0;
+  const int nx = g.nx, ny = g.ny;
+  const long long n = (long long)nx * ny;
+  const bool full_bounds = *a.tape.nan_seen != 0;   // a NaN somewhere: the bounds' comparisons decide
+  for (long long cc = blockIdx.x * (long long)blockDim.x + threadIdx.x; cc < n; cc += (long long)gridDim.x * blockDim.x) {
+    const int c = int(cc);
+    const int i = c % nx, j = c / nx;
+    // away from the sides every index is an offset (the corner one cell below takes
+    // the general rule up to column and row 2, see corner_adjoint)
+    const bool inner = i >= 3 && i < nx - 2 && j >= 3 && j < ny - 2;
+    FaceIdx f;
+    if (inner) {
+      const int on = ydir ? nx : 1;
+      f.a = c;
+      f.b = f.to = c + on;
+      f.am = c - on;
+      f.bp = c + 2 * on;
+      f.axp = c + 1; f.axm = c - 1; f.ayp = c + nx; f.aym = c - nx;
+      f.b_in = true;
+      f.b_own = false;
+    } else {
+      f = face_idx(g, i, j, ydir);
+    }
+    // the face states, normal components first (slots 1, 2 and 4, 5 trade places for
+    // a y face), as phase 2 of the stage kernel makes them
+    const double inv_h = ydir ? g.inv_dy : g.inv_dx, inv_2h = ydir ? g.inv_2dy : g.inv_2dx;
+    const double hh = ydir ? g.hy : g.hx;
+    auto field = [&](int q) { return (q == 1 || q == 4) ? q + d : ((q == 2 || q == 5) ? q - d : q); };
+    auto slope = [&](double lo, double mid, double hi) {
+      if (!g.slope) return (hi - lo) * inv_2h;
+      if (g.limiter == LIMITER_VAN_LEER) return limit_slope<double, LIMITER_VAN_LEER>((mid - lo) * inv_h, (hi - mid) * inv_h);
+      return limit_slope<double, LIMITER_MC>((mid - lo) * inv_h, (hi - mid) * inv_h);
+    };
+    double L[6], Rv[6];
+    unsigned outside = 0;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      const double* s = a.tape.P[field(q)];
+      const double fm = s[f.am], f0 = s[f.a], fp = s[f.b], fpp = s[f.bp];
+      const double fb0 = f.b_own ? fp : f0;   // the high cell's low neighbour in its slope
+      L[q] = f0 + hh * slope(fm, f0, fp);
+      Rv[q] = fp - hh * slope(fb0, fp, fpp);
+      // between the two cells' values (and above the rho / P floor of the bounds):
+      // inside the MOOD bounds
+      const double vlo = (f0 < fp) ? f0 : fp, vhi = (f0 < fp) ? fp : f0;
+      bool in = L[q] >= vlo && L[q] <= vhi && Rv[q] >= vlo && Rv[q] <= vhi;
+      if (q == 0 || q == 3) in = in && L[q] >= 0.1e-8 && Rv[q] >= 0.1e-8;
+      if (!in) outside |= 1u << q;
+    }
+    unsigned toL = 0, toR = 0;      // bit q: the state was reset to the low cell's value
+    unsigned cutL = 0, cutR = 0;    // bit q: a face floor holds
+    if (g.mood && (outside || full_bounds)) {
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const double* s = a.tape.P[field(q)];
+        const double f0 = s[f.a];
+        double lo = dmin(dmin(dmin(dmin(f0, s[f.axp]), s[f.axm]), s[f.ayp]), s[f.aym]);
+        const double hi = dmax(dmax(dmax(dmax(f0, s[f.axp]), s[f.axm]), s[f.ayp]), s[f.aym]);
+        if (q == 0 || q == 3) lo = dmax(0.1e-8, lo);
+        if (L[q] < lo || L[q] > hi) { L[q] = f0; toL |= 1u << q; }
+        if (Rv[q] < lo || Rv[q] > hi) { Rv[q] = f0; toR |= 1u << q; }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 6; q += 3) {
+      if (!(L[q] > 1.0e-8)) { L[q] = 1.0e-8; cutL |= 1u << q; }
+      if (!(Rv[q] > 1.0e-8)) { Rv[q] = 1.0e-8; cutR |= 1u << q; }
+    }
+    const bool coldL = L[3] - 0.5 * (L[4] * L[4] + L[5] * L[5]) < K<double>::P_floor;
+    const bool coldR = Rv[3] - 0.5 * (Rv[4] * Rv[4] + Rv[5] * Rv[5]) < K<double>::P_floor;
+    if (coldL || coldR) {
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const double f0 = a.tape.P[field(q)][f.a];
+        if (coldL) L[q] = f0;
+        if (coldR) Rv[q] = f0;
+      }
+    }
+    if (coldL) { toL = 0x3fu; cutL = 0; }
+    if (coldR) { toR = 0x3fu; cutR = 0; }
+    // adjoint of the face's fluxes: the flux leaves cell a and enters the cell above
+    // (none past an outflow high side)
     double lF[5];
-    const double wgt = ydir ? ay : ax;
-    // the flux leaves cell a and enters cell b (none past an outflow high side)
-    for (int q = 0; q < 4; ++q) lF[q] = wgt * ((f.b_in ? r.lUp[q][f.to] : 0.0) - r.lUp[q][c]);
+    {
+      double lo[4], hi[4] = {0.0, 0.0, 0.0, 0.0};
+      update_adjoint(a, f.a, lo);
+      if (f.b_in) update_adjoint(a, f.to, hi);
+      const double w = a.dt * (ydir ? g.dx : g.dy);
+      const double mx = w * (hi[1] - lo[1]), my = w * (hi[2] - lo[2]);
+      lF[0] = w * (hi[0] - lo[0]);
+      lF[1] = ydir ? my : mx;
+      lF[2] = ydir ? mx : my;
+      lF[3] = w * (hi[3] - lo[3]);
+    }
     // Ez(i,j) = 1/4 (-Fx(i,j) - Fx(i,j+1) + Fy(i,j) + Fy(i+1,j)); at an outflow
     // high side Fx(i,ny) / Fy(nx,j) is the face itself (zero gradient)
-    const double e0 = r.lEz[c];
-    if (!ydir) {
-      double s4 = (j > 0 || g.pyh) ? e0 + r.lEz[wrap(j - 1, g.ny) * g.nx + i] : e0;
-      if (j == g.ny - 1 && !g.pyh) s4 += e0;
-      lF[4] = -0.25 * s4;
-    } else {
-      double s4 = (i > 0 || g.pxh) ? e0 + r.lEz[j * g.nx + wrap(i - 1, g.nx)] : e0;
-      if (i == g.nx - 1 && !g.pxh) s4 += e0;
-      lF[4] = 0.25 * s4;
-    }
-    // recompute the face states (values + flags), then the flux Jacobian
-    double L[6], Rv[6];
-    uint32_t fl;
-    face_states<double>(g, t, f.a, f.b, f.am, f.bp, f.axp, f.axm, f.ayp, f.aym, ydir, f.b_own, L, Rv, &fl);
-    // solver inputs in (normal, tangential) order, seeded 0..11
-    const int perm[6] = {0, ydir ? 2 : 1, ydir ? 1 : 2, 3, ydir ? 5 : 4, ydir ? 4 : 5};  // input slot -> field
-    D in[12];
-    for (int s = 0; s < 6; ++s) {
-      in[2 * s] = seed<12>(L[perm[s]], 2 * s);
-      in[2 * s + 1] = seed<12>(Rv[perm[s]], 2 * s + 1);
-    }
-    Flux5<D> F = riemann<D, SOLVER>(D(g.gamma), in[0], in[1], in[2], in[3], in[4], in[5], in[6], in[7], in[8],
-                                    in[9], in[10], in[11]);
-    // map conserved-ordered lF onto the solver outputs (mass, momn, momt, energy, bt)
-    const double lo_mass = lF[0], lo_mn = ydir ? lF[2] : lF[1], lo_mt = ydir ? lF[1] : lF[2];
-    const double lo_e = lF[3], lo_bt = lF[4];
-    double lL[6] = {0, 0, 0, 0, 0, 0}, lR[6] = {0, 0, 0, 0, 0, 0};
-    for (int s = 0; s < 6; ++s) {
-      for (int side = 0; side < 2; ++side) {
-        const int kk = 2 * s + side;
-        const double v = lo_mass * F.mass.d[kk] + lo_mn * F.momn.d[kk] + lo_mt * F.momt.d[kk] +
-                         lo_e * F.energy.d[kk] + lo_bt * F.bt.d[kk];
-        if (side == 0) lL[perm[s]] += v;
-        else lR[perm[s]] += v;
+    {
+      double s4;
+      if (inner) {
+        const double* lx = a.lout[4];
+        const double* ly = a.lout[5];
+        const int m = ydir ? c - 1 : c - nx;   // the face's other corner
+        const double sx = (lx[c + nx] - lx[c]) + (lx[m + nx] - lx[m]), sy = (ly[c] - ly[c + 1]) + (ly[m] - ly[m + 1]);
+        s4 = a.c1 * (a.dt * g.inv_dy * sx + a.dt * g.inv_dx * sy);
+      } else {
+      const double e0 = corner_adjoint(a, i, j);
+      s4 = e0;
+      if (!ydir) {
+        if (j > 0 || g.pyh) s4 += corner_adjoint(a, i, wrap(j - 1, g.ny));
+        if (j == g.ny - 1 && !g.pyh) s4 += e0;
+      } else {
+        if (i > 0 || g.pxh) s4 += corner_adjoint(a, wrap(i - 1, g.nx), j);
+        if (i == g.nx - 1 && !g.pxh) s4 += e0;
       }
+      }
+      lF[4] = (ydir ? 0.25 : -0.25) * s4;
     }
-    // through the thermal check, face floors and MOOD to cell values and slopes
-    const double hh = ydir ? g.hy : g.hx;
-    double* const* dst = ydir ? r.fY : r.fX;
-    const bool thL = fl & (1u << 24), thR = fl & (1u << 25);
+    double gL[6], gR[6];
+    face_vjp<SOLVER>(g.gamma, g.igm1, L, Rv, lF, gL, gR);
+    // back through the decisions: on through the slope, to the low cell's value, or lost to a floor
+    const unsigned direct = (toL & ~cutL) | (toR & ~cutR);
+    a.fflag[d][c] = direct ? 1 : 0;
+#pragma unroll
     for (int q = 0; q < 6; ++q) {
-      double l_fa = 0.0, l_sa = 0.0, l_fb = 0.0, l_sb = 0.0;
-      if (thL) {
-        l_fa += lL[q];
-      } else if (!(fl & (1u << (4 * q + 2)))) {
-        if (fl & (1u << (4 * q + 0))) l_fa += lL[q];
-        else { l_fa += lL[q]; l_sa += hh * lL[q]; }
-      }
-      if (thR) {
-        l_fa += lR[q];
-      } else if (!(fl & (1u << (4 * q + 3)))) {
-        if (fl & (1u << (4 * q + 1))) l_fa += lR[q];
-        else { l_fb += lR[q]; l_sb -= hh * lR[q]; }
-      }
-      dst[4 * q + 0][c] = l_fa;
-      dst[4 * q + 1][c] = l_sa;
-      dst[4 * q + 2][c] = l_fb;
-      dst[4 * q + 3][c] = l_sb;
+      const unsigned b = 1u << q;
+      a.fL[d][field(q)][c] = ((toL | cutL) & b) ? 0.0 : gL[q];
+      a.fR[d][field(q)][c] = ((toR | cutR) & b) ? 0.0 : gR[q];
+      if (direct) a.fX[d][field(q)][c] = ((toL & ~cutL & b) ? gL[q] : 0.0) + ((toR & ~cutR & b) ? gR[q] : 0.0);
     }
   }
 }
 
-// per cell: gather the slope adjoints from the faces, apply the limiter's
-// local derivative, and gather the direct value adjoints
-__global__ void k_rev_slopes(AdjGeom g, StageTape t, RevBuf r) {
-  const int n = g.nx * g.ny;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    const int i = c % g.nx, j = c / g.nx;
-    // the slope stencil of this cell (each side's ghost rule)
-    const int cxm = j * g.nx + src(i - 1, g.nx, g.px, g.pxh), cym = src(j - 1, g.ny, g.py, g.pyh) * g.nx + i;
-    const int cxp = j * g.nx + src(i + 1, g.nx, g.px, g.pxh), cyp = src(j + 1, g.ny, g.py, g.pyh) * g.nx + i;
-    // the face below this cell, whose high cell it is: none at x = 0 / y = 0
+// The slope's derivative w.r.t. its two one-sided differences dl, dr (times ls, the
+// slope's adjoint), each back to the field: wl for (f0 - fm), wr for (fp - f0).
+// Kink convention where a one-sided difference is exactly zero (a uniform
+// neighbourhood): both zero -> the centred slope's (1/2, 1/2), the limit along
+// dl = dr for MC and Van Leer; one zero -> the mean of the one-sided derivatives,
+// 1 w.r.t. the zero argument (the limiters grow as 2|df| on the active side), 0
+// w.r.t. the other.  Ties of the MC minimum: the mean.
+__device__ __forceinline__ void slope_vjp(const AdjGeom& g, double dl, double dr, double& sl, double& sr) {
+  const double prod = dl * dr, den = dl + dr;
+  sl = sr = 0.0;
+  if (dl == 0.0 || dr == 0.0) {
+    sl = (dl != 0.0) ? 0.0 : ((dr == 0.0) ? 0.5 : 1.0);
+    sr = (dl == 0.0) ? ((dr == 0.0) ? 0.5 : 0.0) : 1.0;
+  } else if (!(prod <= 0.0 || fabs(den) < 1e-12)) {
+    if (g.limiter == LIMITER_VAN_LEER) {
+      const double ib = 1.0 / den, s = (2.0 * prod) * ib;
+      sl = (2.0 * dr - s) * ib;
+      sr = (2.0 * dl - s) * ib;
+    } else {
+      const double x = 2.0 * fabs(dl), y = 2.0 * fabs(dr), z = 0.5 * fabs(den);
+      const double wx = min_weight(x, y), m = (x < y) ? x : y, wm = min_weight(m, z);
+      sl = 2.0 * wx * wm + 0.5 * (1.0 - wm);
+      sr = 2.0 * (1.0 - wx) * wm + 0.5 * (1.0 - wm);
+    }
+  }
+}
+
+__device__ __forceinline__ int wrap_far(int p, int n) {   // any p >= -n
+  while (p < 0) p += n;
+  while (p >= n) p -= n;
+  return p;
+}
+
+constexpr int RC_TX = 32, RC_TY = 8, RC_NT = 352;   // cells of a CTA's tile, threads
+constexpr int RC_EX = RC_TX + 1, RC_EY = RC_TY + 1;   // with the column and the row above, for the face B
+
+// One cell: a CTA takes a 32 x 8 tile and the column and row beyond it, whose cell-B
+// adjoints the tile's face B needs (297 cells on 352 threads).  Field by field, the
+// limiter's derivative of every slope that touches the tile goes to shared memory
+// once (35 x 9 in x, 33 x 11 in y: two a thread, whose indices are formed once) and
+// each cell gathers its own and its neighbours'; fields in pairs (twice the loads in
+// flight) and two buffers, so that three barriers are enough.  Bound by the latency of
+// those loads (long-scoreboard stalls 11 an issue with one field a barrier): two CTAs
+// an SM at 80 registers took 98 us at 512^2 field by field and 70 in pairs, one CTA at
+// 168 registers 30 us more.
+__global__ void __launch_bounds__(RC_NT, 2) k_rev_cells(const __grid_constant__ RevStage a) {
+  constexpr int XW = RC_EX + 2, NX = XW * RC_EY, YW = RC_EX, NY = YW * (RC_EY + 2);
+  constexpr int SLOTS = (NX + NY + RC_NT - 1) / RC_NT;
+  __shared__ double sw[2][2][2][NX + NY];   // [buffer][field of the pair][wl, wr]: x slopes, then y slopes
+  __shared__ double sB[2][RC_EX * RC_EY];
+  const AdjGeom& g = a.g;
+  const int nx = g.nx, ny = g.ny;
+  const unsigned n = unsigned(nx) * unsigned(ny);
+  const int tiles_x = (nx + RC_TX - 1) / RC_TX, tiles_y = (ny + RC_TY - 1) / RC_TY;
+  const int tid = threadIdx.x;
+  for (int tile = blockIdx.x; tile < tiles_x * tiles_y; tile += gridDim.x) {
+    const int i0 = (tile % tiles_x) * RC_TX, j0 = (tile / tiles_x) * RC_TY;
+    // this thread's slopes: the cell, its neighbours in the slope (each side's ghost
+    // rule) and the face below it, if it is that face's high cell
+    // (faces of y at n + cell: the two directions' arrays of a field adjoin)
+    int sk[SLOTS], slo[SLOTS], shi[SLOTS];
+    unsigned sf[SLOTS];
+    bool below[SLOTS];
+#pragma unroll
+    for (int t = 0; t < SLOTS; ++t) {
+      const int e = tid + t * RC_NT;
+      const bool yd = e >= NX;
+      const int ee = yd ? e - NX : e;
+      const int pi = wrap_far(i0 + (yd ? ee % YW : ee % XW - 1), nx), pj = wrap_far(j0 + (yd ? ee / YW - 1 : ee / XW), ny);
+      sk[t] = pj * nx + pi;
+      if (!yd) {
+        slo[t] = pj * nx + src(pi - 1, nx, g.px, g.pxh);
+        shi[t] = pj * nx + src(pi + 1, nx, g.px, g.pxh);
+        below[t] = pi > 0 || g.pxh;
+        sf[t] = unsigned(pj * nx + wrap(pi - 1, nx));
+      } else {
+        slo[t] = src(pj - 1, ny, g.py, g.pyh) * nx + pi;
+        shi[t] = src(pj + 1, ny, g.py, g.pyh) * nx + pi;
+        below[t] = pj > 0 || g.pyh;
+        sf[t] = n + unsigned(wrap(pj - 1, ny) * nx + pi);
+      }
+    }
+    const bool have = tid < RC_EX * RC_EY;
+    const int li = tid % RC_EX, lj = have ? tid / RC_EX : 0;
+    const int i = wrap_far(i0 + li, nx), j = wrap_far(j0 + lj, ny);
+    const int c = j * nx + i;
+    // the faces whose high cell this is: none at x = 0 / y = 0
     // unless the high side wraps to it; past an outflow high side the ghost's
     // value is this cell's (its slope, from two equal differences, depends on
     // no cell)
-    const int fxm = j * g.nx + wrap(i - 1, g.nx), fym = wrap(j - 1, g.ny) * g.nx + i;
-    const bool hx = i > 0 || g.pxh, hy = j > 0 || g.pyh;
-    const bool ex = !g.pxh && i == g.nx - 1, ey = !g.pyh && j == g.ny - 1;
-    for (int q = 0; q < 6; ++q) {
-      // this cell is the low cell of faces (c, x) and (c, y), the high cell of (cxm, x) and (cym, y)
-      double lv = r.fX[4 * q + 0][c] + r.fY[4 * q + 0][c] + (hx ? r.fX[4 * q + 2][fxm] : 0.0) +
-                  (hy ? r.fY[4 * q + 2][fym] : 0.0);
-      if (ex) lv += r.fX[4 * q + 2][c];
-      if (ey) lv += r.fY[4 * q + 2][c];
-      r.lPc[q][c] = lv;
-      for (int d = 0; d < 2; ++d) {
-        const double ls = (d == 0) ? (r.fX[4 * q + 1][c] + (hx ? r.fX[4 * q + 3][fxm] : 0.0))
-                                   : (r.fY[4 * q + 1][c] + (hy ? r.fY[4 * q + 3][fym] : 0.0));
-        const double fm = t.P[q][d == 0 ? cxm : cym], f0 = t.P[q][c], fp = t.P[q][d == 0 ? cxp : cyp];
-        const double inv_h = d == 0 ? g.inv_dx : g.inv_dy;
-        double wl, wr;
-        if (g.slope) {
-          using D2 = Dual<2>;
-          D2 dl = seed<2>((f0 - fm) * inv_h, 0), dr = seed<2>((fp - f0) * inv_h, 1);
-          D2 s = (g.limiter == LIMITER_VAN_LEER) ? limit_slope<D2, LIMITER_VAN_LEER>(dl, dr)
-                                                 : limit_slope<D2, LIMITER_MC>(dl, dr);
-          double dsl = s.d[0], dsr = s.d[1];
-          // Kink convention where a one-sided difference is exactly zero (a
-          // uniform neighbourhood): both zero -> the centred slope's (1/2, 1/2),
-          // the limit along dfL = dfR for MC and Van Leer; one zero -> the mean
-          // of the one-sided derivatives, 1 w.r.t. the zero argument (the
-          // limiters grow as 2|df| on the active side), 0 w.r.t. the other.
-          if (dl.v == 0.0 && dr.v == 0.0) { dsl = 0.5; dsr = 0.5; }
-          else if (dl.v == 0.0) { dsl = 1.0; dsr = 0.0; }
-          else if (dr.v == 0.0) { dsl = 0.0; dsr = 1.0; }
-          wl = ls * dsl * inv_h;
-          wr = ls * dsr * inv_h;
-        } else {
-          const double inv_2h = d == 0 ? g.inv_2dx : g.inv_2dy;
-          wl = ls * inv_2h;
-          wr = ls * inv_2h;
-        }
-        r.w[(q * 2 + d) * 2 + 0][c] = wl;
-        r.w[(q * 2 + d) * 2 + 1][c] = wr;
-      }
-    }
-  }
-}
-
-// per cell: primitive adjoints -> conserved adjoints (+ cell B adjoints)
-__global__ void k_rev_prims(AdjGeom g, StageTape t, RevBuf r, const double* const* __restrict__ Uin,
-                            double* const* __restrict__ lin) {
-  const int n = g.nx * g.ny;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    const int i = c % g.nx, j = c / g.nx;
-    const int cxm = j * g.nx + wrap(i - 1, g.nx), cym = wrap(j - 1, g.ny) * g.nx + i;
-    const int cxp = j * g.nx + wrap(i + 1, g.nx), cyp = wrap(j + 1, g.ny) * g.nx + i;
+    const int fxm = (i > 0 || g.pxh) ? j * nx + wrap(i - 1, nx) : -1;
+    const int fym = (j > 0 || g.pyh) ? wrap(j - 1, ny) * nx + i : -1;
+    const bool ex = !g.pxh && i == nx - 1, ey = !g.pyh && j == ny - 1;
+    const bool resetx = a.fflag[0][c] != 0, resety = a.fflag[1][c] != 0;
     double lP[6];
-    for (int q = 0; q < 6; ++q) {
-      double v = r.lPc[q][c];
-      // slopes: s(p) uses f(p-1), f(p), f(p+1).  At an outflow side the ghost
-      // beyond is this cell: at the low side s(0)'s f(-1) and f(0) terms
-      // cancel to -w1, at the high side s(nx-1)'s f(nx-1) and f(nx) terms to w0
-      for (int d = 0; d < 2; ++d) {
-        const double* w0 = r.w[(q * 2 + d) * 2 + 0];
-        const double* w1 = r.w[(q * 2 + d) * 2 + 1];
-        const bool per = d == 0 ? g.px : g.py, perh = d == 0 ? g.pxh : g.pyh;
-        const int k = d == 0 ? i : j, nk = d == 0 ? g.nx : g.ny;
-        const int cm = d == 0 ? cxm : cym, cp = d == 0 ? cxp : cyp;
-        if (per != perh) {
-          // a mixed pair: this cell's own slope, with its own ghost below / above
-          // where that side is outflow, then the slopes of the cells whose low /
-          // high neighbour it is (across a periodic side, through the wrap)
-          const int wm = d == 0 ? j * g.nx + wrap(i - 1, g.nx) : wrap(j - 1, g.ny) * g.nx + i;
-          const int wp = d == 0 ? j * g.nx + wrap(i + 1, g.nx) : wrap(j + 1, g.ny) * g.nx + i;
-          double own = w0[c] - w1[c];
-          if (k == 0 && !per) own -= w0[c];
-          if (k == nk - 1 && !perh) own += w1[c];
-          v += own;
-          if (k + 1 < nk || per) v -= w0[wp];
-          if (k > 0 || perh) v += w1[wm];
-        } else if (per || (k > 0 && k < nk - 1)) {
-          v += w0[c] - w1[c] - w0[cp] + w1[cm];
-        } else if (k == 0) {
-          v += (-w1[c]) - w0[cp];
-        } else {
-          v += w0[c] + w1[cm];
+#pragma unroll
+    for (int q0 = 0; q0 < 6; q0 += 2) {
+#pragma unroll
+      for (int t = 0; t < SLOTS; ++t) {
+        const int e = tid + t * RC_NT;
+        if (e >= NX + NY) break;
+        const bool yd = e >= NX;
+        const unsigned fk = yd ? n + unsigned(sk[t]) : unsigned(sk[t]);
+        double fm[2], f0[2], fp[2], ls[2];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          const double* P = a.tape.P[q0 + w];
+          fm[w] = P[slo[t]];
+          f0[w] = P[sk[t]];
+          fp[w] = P[shi[t]];
+          ls[w] = a.fL[0][q0 + w][fk] - (below[t] ? a.fR[0][q0 + w][sf[t]] : 0.0);
+        }
+        // the slope moves a face state by half a spacing, and its differences are over
+        // a whole one (unlimited: two): factors 1/2 and 1/4 in all
+        const double inv_h = yd ? g.inv_dy : g.inv_dx;
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          double sl = 0.5, sr = 0.5;
+          if (g.slope)
+            slope_vjp(g, (f0[w] - fm[w]) * inv_h, (fp[w] - f0[w]) * inv_h, sl, sr);
+          sw[(q0 >> 1) & 1][w][0][e] = 0.5 * ls[w] * sl;
+          sw[(q0 >> 1) & 1][w][1][e] = 0.5 * ls[w] * sr;
         }
       }
-      lP[q] = v;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        if (!have) break;
+        const int q = q0 + w;
+        const double* const wl = sw[(q0 >> 1) & 1][w][0];
+        const double* const wr = sw[(q0 >> 1) & 1][w][1];
+        // this cell is the low cell of faces (c, x) and (c, y), the high cell of (fxm, x) and (fym, y)
+        double v = a.fL[0][q][c] + a.fL[1][q][c];
+        if (resetx) v += a.fX[0][q][c];
+        if (resety) v += a.fX[1][q][c];
+        if (fxm >= 0) v += a.fR[0][q][fxm];
+        if (fym >= 0) v += a.fR[1][q][fym];
+        if (ex) v += a.fR[0][q][c];
+        if (ey) v += a.fR[1][q][c];
+        // slopes: s(p) uses f(p-1), f(p), f(p+1).  The cell's own slope, with its own
+        // ghost below / above where that side is outflow, then the slopes of the cells
+        // whose low / high neighbour it is (across a periodic side, through the wrap)
+#pragma unroll
+        for (int dd = 0; dd < 2; ++dd) {
+          const int at = dd ? NX + (lj + 1) * YW + li : lj * XW + li + 1, step = dd ? YW : 1;
+          const bool per = dd ? g.py : g.px, perh = dd ? g.pyh : g.pxh;
+          const int k = dd ? j : i, nk = dd ? ny : nx;
+          v += ((k == 0 && !per) ? 0.0 : wl[at]) - ((k == nk - 1 && !perh) ? 0.0 : wr[at]);
+          if (k + 1 < nk || per) v -= wl[at + step];
+          if (k > 0 || perh) v += wr[at - step];
+        }
+        lP[q] = v;
+      }
     }
-    lP[4] += r.lBc[0][c];
-    lP[5] += r.lBc[1][c];
-    for (int q = 0; q < 6; ++q) lP[q] += r.lPcor[q][c];
-    using D = Dual<6>;
-    const double Bx = t.P[4][c], By = t.P[5][c];
-    D M = seed<6>(Uin[0][c], 0), Mx = seed<6>(Uin[1][c], 1), My = seed<6>(Uin[2][c], 2);
-    D E = seed<6>(Uin[3][c], 3), bx = seed<6>(Bx, 4), by = seed<6>(By, 5);
-    Prim<D> p = get_primitive<D>(M, Mx, My, E, bx, by, D(g.gamma), D(g.vol));
-    const D* o[4] = {&p.rho, &p.vx, &p.vy, &p.P};
-    double lv[6];
-    for (int k = 0; k < 6; ++k) {
-      double s = 0.0;
-      for (int q = 0; q < 4; ++q) s += lP[q] * o[q]->d[k];
-      lv[k] = s;
+    // primitives -> conserved (get_primitive transposed), and the cell B
+    double lup[4], lbl[4], lin[4];
+    if (have) {
+      const unsigned hit = a.tape.hit[c];
+      if (hit || (!g.px && i == 0) || (!g.py && j == 0)) {
+        double u4[4], b4[4], lB[2], lcor[6];
+        cell_adjoint_slow(a, c, u4, b4, lB, lcor);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) { lup[q] = u4[q]; lbl[q] = b4[q]; }
+        lP[4] += lB[0];
+        lP[5] += lB[1];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) lP[q] += lcor[q];
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          lbl[q] = a.lout[q][c];
+          lup[q] = a.c1 * lbl[q];
+        }
+      }
+      const double r = a.tape.P[0][c], u = a.tape.P[1][c], v = a.tape.P[2][c];
+      const double Bx = a.tape.P[4][c], By = a.tape.P[5][c];
+      const double gm1 = g.gamma - 1.0, hB = 0.5 * (Bx * Bx + By * By), vv = u * u + v * v, ke = 0.5 * r * vv;
+      const double P0 = ((a.U[3][c] * g.ivol - ke) - hB) * gm1 + hB;
+      const bool warm = P0 > K<double>::P_floor;
+      const double P1 = warm ? P0 : K<double>::P_floor;
+      const double X = hB + K<double>::e_floor_frac * (ke + hB);
+      const double wP = max_weight(P1, X);
+      const double aX = (1.0 - wP) * lP[3], a0 = warm ? wP * lP[3] : 0.0;
+      const double ake = K<double>::e_floor_frac * aX - a0 * gm1;
+      const double ahB = (1.0 + K<double>::e_floor_frac) * aX + a0 * (1.0 - gm1);
+      const double ir = 1.0 / r, im = ir * g.ivol;
+      const double au = lP[1] + ake * r * u, av = lP[2] + ake * r * v;
+      const double ar = lP[0] + ake * (0.5 * vv) - (au * u + av * v) * ir;
+      lin[0] = (a.U[0][c] * g.ivol > K<double>::rho_floor) ? ar * g.ivol : 0.0;
+      lin[1] = au * im;
+      lin[2] = av * im;
+      lin[3] = a0 * gm1 * g.ivol;
+      sB[0][tid] = lP[4] + ahB * Bx;
+      sB[1][tid] = lP[5] + ahB * By;
     }
-    for (int q = 0; q < 4; ++q) lin[q][c] = r.lUp[q][c] + lv[q];   // identity path of the update
-    r.lB2[0][c] = lP[4] + lv[4];
-    r.lB2[1][c] = lP[5] + lv[5];
+    __syncthreads();
+    if (have && li < RC_TX && lj < RC_TY && i0 + li < nx && j0 + lj < ny) {
+      // face B: the CT identity and the two cell averages it enters: b_x(i) enters Bx(i)
+      // (alone at an outflow low side) and Bx(i+1) (none past the high side)
+      const double o4 = a.lout[4][c], o5 = a.lout[5][c];
+      double l[6];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) l[q] = lup[q] + lin[q];
+      l[4] = a.c1 * o4 + ((i > 0 || g.px) ? 0.5 : 1.0) * sB[0][tid] +
+             ((i + 1 < nx || g.px) ? 0.5 * sB[0][tid + 1] : 0.0);
+      l[5] = a.c1 * o5 + ((j > 0 || g.py) ? 0.5 : 1.0) * sB[1][tid] +
+             ((j + 1 < ny || g.py) ? 0.5 * sB[1][tid + RC_EX] : 0.0);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const double b = (q < 4) ? lbl[q < 4 ? q : 0] : (q == 4 ? o4 : o5);
+        if (a.stage == 3) a.lU0[q][c] = a.c0 * b;
+        else if (a.stage == 2) a.lU0[q][c] += a.c0 * b;
+        else l[q] += a.lU0[q][c];
+        a.lin[q][c] = l[q];
+      }
+    }
+    __syncthreads();   // the shared arrays are reused by the next tile
   }
 }
 
-// per cell: face B adjoint = CT identity + the two cell averages it enters
-__global__ void k_rev_faceB(AdjGeom g, RevBuf r, double* const* __restrict__ lin) {
-  const int n = g.nx * g.ny;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    const int i = c % g.nx, j = c / g.nx;
-    const int cxp = j * g.nx + wrap(i + 1, g.nx), cyp = wrap(j + 1, g.ny) * g.nx + i;
-    // b_x(i) enters Bx(i) (alone at an outflow low side) and Bx(i+1) (none past the high side)
-    lin[4][c] = r.lbp[0][c] + ((i > 0 || g.px) ? 0.5 : 1.0) * r.lB2[0][c] +
-                ((i + 1 < g.nx || g.px) ? 0.5 * r.lB2[0][cxp] : 0.0);
-    lin[5][c] = r.lbp[1][c] + ((j > 0 || g.py) ? 0.5 : 1.0) * r.lB2[1][c] +
-                ((j + 1 < g.ny || g.py) ? 0.5 * r.lB2[1][cyp] : 0.0);
-  }
-}
-
-__global__ void k_axpy6(double* const* __restrict__ y, const double* const* __restrict__ x, int n) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-    for (int q = 0; q < 6; ++q) y[q][c] += x[q][c];
-}
-
-__global__ void k_zero6(double* const* __restrict__ y, int n) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-    for (int q = 0; q < 6; ++q) y[q][c] = 0.0;
-}
+// Per-call descriptors of the stage kernels in device memory: one upload a call.
+struct StepDesc {
+  Member member;
+  Control ctl;
+  TapeOut tape[3];
+  int nan_seen;
+};
 
 }  // namespace
 
@@ -644,27 +627,83 @@ struct chimera_adjoint {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   int n = 0;
-  int grid = 0;
+  int sms = 148;
+  KernelSet forward, taped;        // the fused stage kernels without and with the tape
+  int grid_forward[3] = {}, grid_taped[3] = {};
+  Member member;                   // without its buffers and tiling
   double* pool = nullptr;
-  StageTape tape[3];
-  RevBuf rev;
+  TapeOut tape[3];
+  double* fL[2][6];
+  double* fR[2][6];
+  double* fX[2][6];
+  unsigned char* fflag[2];
   double* U1[6];
   double* U2[6];
   double* lA[6];     // stage adjoint buffers
   double* lB[6];
   double* lU0[6];    // accumulated U^n adjoint from the blends
-  double** dptrs = nullptr;   // device copies of pointer arrays
+  StepDesc* desc = nullptr;   // device
 };
-
-namespace {
-// device pointer-array slots
-enum { P_UN = 0, P_U1 = 6, P_U2 = 12, P_LA = 18, P_LB = 24, P_LU0 = 30, P_LNEXT = 36, P_LOUT = 42, P_UNEXT = 48,
-       P_COUNT = 54 };
-}
 
 static int adj_fail() {
   cudaGetLastError();
   return CHIMERA_ERR_CUDA;
+}
+
+static int resident_ctas(const chimera_adjoint* a, const KernelEntry& k) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.nt, k.smem) != cudaSuccess || per_sm < 1)
+    per_sm = 1;
+  cudaGetLastError();
+  return per_sm * a->sms;
+}
+
+static int tiles_of(const chimera_adjoint* a, const KernelEntry& k) {
+  return ((a->g.nx + k.tx - 1) / k.tx) * ((a->g.ny + k.ty - 1) / k.ty);
+}
+
+// The stage kernels of this grid: 8 x 8 tiles where the device holds all of them at
+// once, else 32 x 16, as the solver's handles choose them (their TMA tiles need
+// tensor maps of the caller's arrays; plain loads here).
+static void pick_kernels(chimera_adjoint* a, bool mixed) {
+  auto allow = [&](KernelSet& ks) {
+    for (int s = 0; s < 3; ++s)
+      cudaFuncSetAttribute(ks.stage[a->g.riemann - 1][s].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           int(ks.stage[a->g.riemann - 1][s].smem));
+    cudaGetLastError();
+  };
+  auto fits = [&](const KernelSet& ks) {
+    for (int s = 0; s < 3; ++s) {
+      const KernelEntry& k = ks.stage[a->g.riemann - 1][s];
+      if (tiles_of(a, k) > resident_ctas(a, k)) return false;
+    }
+    return true;
+  };
+  auto grids = [&](const KernelSet& ks, int* grid) {
+    for (int s = 0; s < 3; ++s) {
+      const KernelEntry& k = ks.stage[a->g.riemann - 1][s];
+      grid[s] = std::max(1, std::min(tiles_of(a, k), resident_ctas(a, k)));
+    }
+  };
+  if (mixed) {
+    fp64_mixed_pair_kernels(&a->forward);
+    tape_mixed_pair_kernels(&a->taped);
+  } else {
+    bool found = false;
+    for (int v : {7, 8, 9}) {   // the small-grid variants
+      fp64_kernels(v, &a->forward);
+      allow(a->forward);
+      if ((found = fits(a->forward))) break;
+    }
+    if (!found) fp64_kernels(1, &a->forward);
+    tape_kernels(true, &a->taped);
+    allow(a->taped);
+    if (!fits(a->taped)) tape_kernels(false, &a->taped);
+  }
+  allow(a->forward);
+  allow(a->taped);
+  grids(a->forward, a->grid_forward);
+  grids(a->taped, a->grid_taped);
 }
 
 extern "C" int chimera_adjoint_create(const chimera_cfg* cfg, void* stream, chimera_adjoint** out) {
@@ -688,6 +727,8 @@ extern "C" int chimera_adjoint_create(const chimera_cfg* cfg, void* stream, chim
   g.hx = 0.5 * cfg->dx; g.hy = 0.5 * cfg->dy;
   g.gamma = cfg->gamma;
   g.vol = cfg->dx * cfg->dy;
+  g.igm1 = 1.0 / (cfg->gamma - 1.0);
+  g.ivol = 1.0 / g.vol;
   g.riemann = cfg->riemann; g.limiter = cfg->limiter;
   g.slope = cfg->use_slope_limiting ? 1 : 0;
   g.mood = cfg->mood ? 1 : 0;
@@ -701,52 +742,54 @@ extern "C" int chimera_adjoint_create(const chimera_cfg* cfg, void* stream, chim
     if (cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking) != cudaSuccess) { delete a; return adj_fail(); }
     a->own_stream = true;
   }
-  int dev = 0, sms = 148;
+  int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaDeviceGetAttribute(&a->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
     cudaGetLastError();
-    sms = 148;
+    a->sms = 148;
   }
-  a->grid = sms * 8;
-  // doubles per cell: tapes 3 x (6 P + 10 F + 4 Upre + 4 Ublend) + 2 flag words (as 1 double)
-  // + reverse (4 + 2 + 2 + 1 + 48 + 24 + 6 + 2 + 6) + U1, U2, lA, lB, lU0 (30)
-  const size_t per_cell = 3 * (24 + 1) + (4 + 2 + 2 + 1 + 48 + 24 + 6 + 2 + 6) + 30;
-  const size_t n = size_t(a->n);
-  if (cudaMalloc(&a->pool, per_cell * n * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&a->dptrs, P_COUNT * sizeof(double*)) != cudaSuccess) {
+  Member& m = a->member;
+  memset(&m, 0, sizeof(m));
+  m.nx = g.nx; m.ny = g.ny;
+  m.periodic_x = g.px; m.periodic_y = g.py;
+  m.periodic_xhi = g.pxh; m.periodic_yhi = g.pyh;
+  m.square = (cfg->dx == cfg->dy) ? 1 : 0;
+  m.dx = g.dx; m.dy = g.dy;
+  m.inv_dx = g.inv_dx; m.inv_dy = g.inv_dy;
+  m.inv_2dx = g.inv_2dx; m.inv_2dy = g.inv_2dy;
+  m.hx = g.hx; m.hy = g.hy;
+  m.gamma = g.gamma;
+  m.vol = g.vol;
+  m.len = (cfg->dx < cfg->dy) ? cfg->dx : cfg->dy;
+  m.inv_vol = 1.0 / g.vol;
+  m.rcp_vol = shared_reciprocal(g.vol);
+  m.rcp_gm1 = shared_reciprocal(g.gamma - 1.0);
+  pick_kernels(a, g.px != g.pxh || g.py != g.pyh);
+  // doubles per cell: tapes 3 x (6 P + 4 Upre + 4 Ublend), faces 2 x 18, U1, U2, lA, lB, lU0 (30);
+  // bytes: 3 floor marks and 2 face flags
+  const size_t n = size_t(a->n), per_cell = 3 * 14 + 2 * 18 + 30;
+  if (cudaMalloc(&a->pool, per_cell * n * sizeof(double) + 5 * n) != cudaSuccess ||
+      cudaMalloc(&a->desc, sizeof(StepDesc)) != cudaSuccess) {
     cudaGetLastError();
     chimera_adjoint_destroy(a);
     return CHIMERA_ERR_NOMEM;
   }
   double* p = a->pool;
   auto take = [&]() { double* r = p; p += n; return r; };
-  for (int k = 0; k < 3; ++k) {
-    StageTape& t = a->tape[k];
+  for (TapeOut& t : a->tape) {
     for (int q = 0; q < 6; ++q) t.P[q] = take();
-    for (int q = 0; q < 5; ++q) t.Fx[q] = take();
-    for (int q = 0; q < 5; ++q) t.Fy[q] = take();
     for (int q = 0; q < 4; ++q) t.Upre[q] = take();
     for (int q = 0; q < 4; ++q) t.Ublend[q] = take();
-    uint32_t* fw = reinterpret_cast<uint32_t*>(take());   // 2 x n flag words in n doubles
-    t.flx = fw;
-    t.fly = fw + n;
+    t.nan_seen = &a->desc->nan_seen;
   }
-  RevBuf& r = a->rev;
-  for (int q = 0; q < 4; ++q) r.lUp[q] = take();
-  for (int q = 0; q < 2; ++q) r.lBc[q] = take();
-  for (int q = 0; q < 2; ++q) r.lbp[q] = take();
-  r.lEz = take();
-  for (int q = 0; q < 24; ++q) r.fX[q] = take();
-  for (int q = 0; q < 24; ++q) r.fY[q] = take();
-  for (int q = 0; q < 24; ++q) r.w[q] = take();
-  for (int q = 0; q < 6; ++q) r.lPc[q] = take();
-  for (int q = 0; q < 2; ++q) r.lB2[q] = take();
-  for (int q = 0; q < 6; ++q) r.lPcor[q] = take();
-  for (int q = 0; q < 6; ++q) a->U1[q] = take();
-  for (int q = 0; q < 6; ++q) a->U2[q] = take();
-  for (int q = 0; q < 6; ++q) a->lA[q] = take();
-  for (int q = 0; q < 6; ++q) a->lB[q] = take();
-  for (int q = 0; q < 6; ++q) a->lU0[q] = take();
+  for (auto* f : {a->fL, a->fR, a->fX})
+    for (int q = 0; q < 6; ++q)
+      for (int d = 0; d < 2; ++d) f[d][q] = take();   // (a field's two directions adjoin)
+  for (auto* f : {a->U1, a->U2, a->lA, a->lB, a->lU0})
+    for (int q = 0; q < 6; ++q) f[q] = take();
+  unsigned char* b = reinterpret_cast<unsigned char*>(p);
+  for (TapeOut& t : a->tape) { t.hit = b; b += n; }
+  for (int d = 0; d < 2; ++d) { a->fflag[d] = b; b += n; }
   *out = a;
   return CHIMERA_OK;
 }
@@ -755,69 +798,112 @@ extern "C" void chimera_adjoint_destroy(chimera_adjoint* a) {
   if (!a) return;
   if (a->stream) cudaStreamSynchronize(a->stream);
   cudaFree(a->pool);
-  cudaFree(a->dptrs);
+  cudaFree(a->desc);
   if (a->own_stream && a->stream) cudaStreamDestroy(a->stream);
   cudaGetLastError();
   delete a;
 }
 
-// Upload the pointer arrays a launch needs (one H2D copy per call).
-static int upload_ptrs(chimera_adjoint* a, const double* const* Un, const double* const* lnext, double* const* lout,
-                       double* const* Unext) {
-  double* h[P_COUNT];
-  memset(h, 0, sizeof(h));
+// The three stages from U_n on the stage kernels ks.  Taped: U1 and U2 stay in the
+// handle's buffers and U_{n+1} is not written.  Else U_{n+1} goes to out, which
+// serves as U1 on the way.  Control is the same for all three: dry launches leave
+// it alone.
+static int run_stages(chimera_adjoint* a, const KernelSet& ks, const int* grid, double dt, const double* const* U_n,
+                      double* const* out, bool taped) {
+  StepDesc d;
+  memset(&d, 0, sizeof(d));
+  d.member = a->member;
+  const KernelEntry& k0 = ks.stage[a->g.riemann - 1][0];
+  d.member.tiles_x = (a->g.nx + k0.tx - 1) / k0.tx;
+  d.member.tiles_y = (a->g.ny + k0.ty - 1) / k0.ty;
   for (int q = 0; q < 6; ++q) {
-    h[P_UN + q] = const_cast<double*>(Un ? Un[q] : nullptr);
-    h[P_U1 + q] = a->U1[q];
-    h[P_U2 + q] = a->U2[q];
-    h[P_LA + q] = a->lA[q];
-    h[P_LB + q] = a->lB[q];
-    h[P_LU0 + q] = a->lU0[q];
-    h[P_LNEXT + q] = const_cast<double*>(lnext ? lnext[q] : nullptr);
-    h[P_LOUT + q] = lout ? lout[q] : nullptr;
-    h[P_UNEXT + q] = Unext ? Unext[q] : nullptr;
+    d.member.buf[0][q] = const_cast<double*>(U_n[q]);
+    d.member.buf[1][q] = taped ? a->U1[q] : out[q];
+    d.member.buf[2][q] = a->U2[q];
   }
-  if (cudaMemcpyAsync(a->dptrs, h, sizeof(h), cudaMemcpyHostToDevice, a->stream) != cudaSuccess) return adj_fail();
+  d.ctl.dt = dt;
+  d.ctl.active = 1;
+  d.ctl.output_count = 1;
+  for (int s = 0; s < 3; ++s) d.tape[s] = a->tape[s];
+  if (cudaMemcpyAsync(a->desc, &d, sizeof(d), cudaMemcpyHostToDevice, a->stream) != cudaSuccess) return adj_fail();
+  StageArgs s;
+  memset(&s, 0, sizeof(s));
+  s.members = &a->desc->member;
+  s.ctl = &a->desc->ctl;
+  s.n_members = 1;
+  s.total_tiles = d.member.tiles_x * d.member.tiles_y;
+  s.limiter = a->g.limiter;
+  s.slope_limiting = a->g.slope;
+  s.mood = a->g.mood;
+  s.dry = 1;
+  for (int k = 0; k < 3; ++k) {
+    const KernelEntry& e = ks.stage[a->g.riemann - 1][k];
+    s.tape = taped ? &a->desc->tape[k] : nullptr;
+    void* args[] = {&s};
+    // a stage's launch overlaps the end of the one before it (grid_wait in the kernels)
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid[k]);
+    cfg.blockDim = dim3(e.nt);
+    cfg.dynamicSmemBytes = e.smem;
+    cfg.stream = a->stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = k > 0 ? 1 : 0;
+    if (cudaLaunchKernelExC(&cfg, e.fn, args) != cudaSuccess) return adj_fail();
+  }
   return CHIMERA_OK;
 }
 
-template <int SOLVER>
-static void tape_stage(chimera_adjoint* a, int stage, double dt, double** in, double** u0, double** out) {
-  const int grid = a->grid;
-  StageTape& t = a->tape[stage - 1];
-  k_tape_prims<<<grid, 256, 0, a->stream>>>(a->g, in, t);
-  k_tape_faces<SOLVER><<<grid, 128, 0, a->stream>>>(a->g, t);
-  k_tape_update<<<grid, 256, 0, a->stream>>>(a->g, stage, dt, in, u0, t, out);
+// One stage of the reverse sweep from input U and output adjoint lout to lin.
+static void rev_stage(chimera_adjoint* a, int stage, double dt, const double* const* U, const double* const* lout,
+                      double* const* lin) {
+  RevStage r;
+  r.g = a->g;
+  r.stage = stage;
+  r.dt = dt;
+  r.c0 = (stage == 1) ? 0.0 : ((stage == 2) ? 0.75 : 1.0 / 3.0);
+  r.c1 = (stage == 1) ? 1.0 : ((stage == 2) ? 0.25 : 2.0 / 3.0);
+  r.tape = a->tape[stage - 1];
+  for (int q = 0; q < 6; ++q) {
+    r.U[q] = U[q];
+    r.lout[q] = lout[q];
+    r.lin[q] = lin[q];
+    r.lU0[q] = a->lU0[q];
+    for (int d = 0; d < 2; ++d) {
+      r.fL[d][q] = a->fL[d][q];
+      r.fR[d][q] = a->fR[d][q];
+      r.fX[d][q] = a->fX[d][q];
+    }
+  }
+  for (int d = 0; d < 2; ++d) r.fflag[d] = a->fflag[d];
+  const dim3 faces(unsigned(std::min<long long>((a->n + 127) / 128, 1 << 20)), 2);
+  switch (a->g.riemann) {
+    case CHIMERA_RIEMANN_RUSANOV: k_rev_faces<RIEMANN_RUSANOV><<<faces, 128, 0, a->stream>>>(r); break;
+    case CHIMERA_RIEMANN_HLLE: k_rev_faces<RIEMANN_HLLE><<<faces, 128, 0, a->stream>>>(r); break;
+    default: k_rev_faces<RIEMANN_HLLD><<<faces, 128, 0, a->stream>>>(r); break;
+  }
+  const long long tiles = (long long)((a->g.nx + RC_TX - 1) / RC_TX) * ((a->g.ny + RC_TY - 1) / RC_TY);
+  k_rev_cells<<<unsigned(std::min<long long>(tiles, 1 << 20)), RC_NT, 0, a->stream>>>(r);
 }
 
-template <int SOLVER>
-static void rev_stage(chimera_adjoint* a, int stage, double dt, double** in, double** lout, double** lin,
-                      double** lU0) {
-  const int grid = a->grid;
-  StageTape& t = a->tape[stage - 1];
-  k_rev_cells1<<<grid, 256, 0, a->stream>>>(a->g, stage, dt, t, lout, a->rev, lU0);
-  k_rev_corners<<<grid, 256, 0, a->stream>>>(a->g, dt, a->rev);
-  k_rev_faces<SOLVER><<<grid, 64, 0, a->stream>>>(a->g, dt, t, a->rev);
-  k_rev_slopes<<<grid, 128, 0, a->stream>>>(a->g, t, a->rev);
-  k_rev_prims<<<grid, 128, 0, a->stream>>>(a->g, t, a->rev, in, lin);
-  k_rev_faceB<<<grid, 256, 0, a->stream>>>(a->g, a->rev, lin);
+// Whether any of the six output arrays overlaps one of the six inputs.
+static bool overlaps(const chimera_adjoint* a, const double* const* in, double* const* out) {
+  const uintptr_t bytes = uintptr_t(a->n) * sizeof(double);
+  for (int p = 0; p < 6; ++p)
+    for (int q = 0; q < 6; ++q) {
+      const uintptr_t x = reinterpret_cast<uintptr_t>(in[p]), y = reinterpret_cast<uintptr_t>(out[q]);
+      if (x < y + bytes && y < x + bytes) return true;
+    }
+  return false;
 }
 
-template <int SOLVER>
-static void forward_step(chimera_adjoint* a, double dt, double** d) {
-  tape_stage<SOLVER>(a, 1, dt, d + P_UN, d + P_UN, d + P_U1);
-  tape_stage<SOLVER>(a, 2, dt, d + P_U1, d + P_UN, d + P_U2);
-  tape_stage<SOLVER>(a, 3, dt, d + P_U2, d + P_UN, d + P_UNEXT);
-}
-
-template <int SOLVER>
-static void adjoint_step(chimera_adjoint* a, double dt, double** d) {
-  forward_step<SOLVER>(a, dt, d);
-  k_zero6<<<a->grid, 256, 0, a->stream>>>(d + P_LU0, a->n);
-  rev_stage<SOLVER>(a, 3, dt, d + P_U2, d + P_LNEXT, d + P_LA, d + P_LU0);   // lambda_U2 -> lA
-  rev_stage<SOLVER>(a, 2, dt, d + P_U1, d + P_LA, d + P_LB, d + P_LU0);      // lambda_U1 -> lB
-  rev_stage<SOLVER>(a, 1, dt, d + P_UN, d + P_LB, d + P_LOUT, d + P_LU0);    // direct lambda_Un
-  k_axpy6<<<a->grid, 256, 0, a->stream>>>(d + P_LOUT, d + P_LU0, a->n);
+static int copy6(chimera_adjoint* a, double* const* dst, double* const* src) {
+  for (int q = 0; q < 6; ++q)
+    if (cudaMemcpyAsync(dst[q], src[q], size_t(a->n) * sizeof(double), cudaMemcpyDeviceToDevice, a->stream) != cudaSuccess)
+      return adj_fail();
+  return CHIMERA_OK;
 }
 
 extern "C" int chimera_adjoint_step(chimera_adjoint* a, const double* const* U_n, double dt,
@@ -825,14 +911,15 @@ extern "C" int chimera_adjoint_step(chimera_adjoint* a, const double* const* U_n
   if (!a || !U_n || !lambda_next || !lambda_n || !(dt > 0.0)) return CHIMERA_ERR_BAD_ARG;
   for (int q = 0; q < 6; ++q)
     if (!doubles_ok({U_n[q], lambda_next[q], lambda_n[q]})) return CHIMERA_ERR_BAD_ARG;
-  // U_{n+1} of the tape forward is not needed: write it into the stage-1 adjoint buffer
-  int rc = upload_ptrs(a, U_n, lambda_next, lambda_n, a->lA);
+  int rc = run_stages(a, a->taped, a->grid_taped, dt, U_n, nullptr, true);
   if (rc) return rc;
-  switch (a->g.riemann) {
-    case CHIMERA_RIEMANN_RUSANOV: adjoint_step<RIEMANN_RUSANOV>(a, dt, a->dptrs); break;
-    case CHIMERA_RIEMANN_HLLE: adjoint_step<RIEMANN_HLLE>(a, dt, a->dptrs); break;
-    default: adjoint_step<RIEMANN_HLLD>(a, dt, a->dptrs); break;
-  }
+  // lambda_n may be U_n's memory: the last stage reads U_n around the cells it writes
+  const bool aside = overlaps(a, U_n, lambda_n);
+  double* const* dst = aside ? a->lA : lambda_n;
+  rev_stage(a, 3, dt, a->U2, lambda_next, a->lA);   // lambda_U2 -> lA
+  rev_stage(a, 2, dt, a->U1, a->lA, a->lB);         // lambda_U1 -> lB
+  rev_stage(a, 1, dt, U_n, a->lB, dst);             // lambda_Un, with the blends' share
+  if (aside && (rc = copy6(a, lambda_n, a->lA))) return rc;
   if (cudaGetLastError() != cudaSuccess) return CHIMERA_ERR_CUDA;
   if (cudaStreamSynchronize(a->stream) != cudaSuccess) return adj_fail();
   return CHIMERA_OK;
@@ -843,13 +930,11 @@ extern "C" int chimera_adjoint_forward_step(chimera_adjoint* a, const double* co
   if (!a || !U_n || !U_next || !(dt > 0.0)) return CHIMERA_ERR_BAD_ARG;
   for (int q = 0; q < 6; ++q)
     if (!doubles_ok({U_n[q], U_next[q]})) return CHIMERA_ERR_BAD_ARG;
-  int rc = upload_ptrs(a, U_n, nullptr, nullptr, U_next);
+  // U_next may be U_n's memory: the stages read U_n around the cells they write
+  const bool aside = overlaps(a, U_n, U_next);
+  int rc = run_stages(a, a->forward, a->grid_forward, dt, U_n, aside ? a->U1 : U_next, false);
   if (rc) return rc;
-  switch (a->g.riemann) {
-    case CHIMERA_RIEMANN_RUSANOV: forward_step<RIEMANN_RUSANOV>(a, dt, a->dptrs); break;
-    case CHIMERA_RIEMANN_HLLE: forward_step<RIEMANN_HLLE>(a, dt, a->dptrs); break;
-    default: forward_step<RIEMANN_HLLD>(a, dt, a->dptrs); break;
-  }
+  if (aside && (rc = copy6(a, U_next, a->U1))) return rc;
   if (cudaGetLastError() != cudaSuccess) return CHIMERA_ERR_CUDA;
   if (cudaStreamSynchronize(a->stream) != cudaSuccess) return adj_fail();
   return CHIMERA_OK;

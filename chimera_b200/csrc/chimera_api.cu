@@ -243,6 +243,7 @@ static int launch_raw(chimera_handle* h, const KernelEntry& k, int grid, int w_b
   a.mood = h->mood;
   a.counters = h->counters;
   a.dry = h->dry;
+  a.tape = nullptr;
   void* args[] = {&a};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);

@@ -65,6 +65,18 @@ struct Control {
   double cfl_speed, divb_max, divb_sum, bmax, mass, energy;
 };
 
+// What a TAPE stage kernel records for the adjoint, per cell: the stage
+// primitives (rho, vx, vy, P_total, Bx, By), which floors changed it (bit 0: the
+// floors after the flux update, bit 1: those after the RK blend), and at such
+// cells only the values that went into them.
+struct TapeOut {
+  double* P[6];
+  double* Upre[4];
+  double* Ublend[4];
+  unsigned char* hit;
+  int* nan_seen;           // set if a primitive is NaN or infinite
+};
+
 struct StageArgs {
   const Member* members;
   Control* ctl;
@@ -76,6 +88,7 @@ struct StageArgs {
   int limiter, slope_limiting, mood;
   int counters;            // count MOOD resets / floor hits
   int dry;                 // timing run: write scratch only, leave Control untouched
+  const TapeOut* tape;     // TAPE kernels only
 };
 
 }  // namespace chimera

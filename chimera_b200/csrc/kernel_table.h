@@ -22,6 +22,9 @@ struct KernelSet {
 int fp64_variant_count();
 void fp64_kernels(int variant, KernelSet* out);
 void fp64_mixed_pair_kernels(KernelSet* out);
+// The FP64 stage kernels that record the adjoint's tape (no CFL kernel).
+void tape_kernels(bool small, KernelSet* out);
+void tape_mixed_pair_kernels(KernelSet* out);
 void fp32_mixed_pair_kernels(KernelSet* out);
 void fp32m_mixed_pair_kernels(KernelSet* out);
 int fp32_variant_count();

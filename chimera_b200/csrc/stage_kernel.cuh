@@ -35,7 +35,7 @@ namespace chimera {
 // symbol -- compiled in two units would give two device bodies under one name,
 // of which a launch runs whichever module the runtime resolved the name to.
 // Each unit passes its own value, so every instantiation is defined once.
-enum { UNIT_FP64 = 0, UNIT_FP32 = 1, UNIT_NOALLOC = 2 };
+enum { UNIT_FP64 = 0, UNIT_FP32 = 1, UNIT_NOALLOC = 2, UNIT_TAPE = 3 };
 
 // A pointer read from global memory where it is used (inline PTX, so that the
 // compiler neither hoists the read nor merges it with an earlier one): keeps
@@ -319,9 +319,11 @@ __device__ void member_finish(const Member& g, Control* ctl, const double* part,
 // face and corner values computed in the halo must be the ones the owning
 // tile computes; the checks cost instructions on every face, so grids without
 // a mixed pair run the MIXBC = false instantiations.
+// TAPE: the adjoint's forward re-run; the stage's primitives and what its floors
+// changed are recorded (TapeOut); stage 3 writes nothing else.
 // ----------------------------------------------------------------------------
 template <typename R, int SOLVER, int STAGE, int TX, int TY, int NT, int MINB, bool KEEP_IN = false,
-          bool TMA = false, int UNIT = UNIT_FP64, bool MIXBC = false>
+          bool TMA = false, int UNIT = UNIT_FP64, bool MIXBC = false, bool TAPE = false>
 __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
   using G = TileGeom<TX, TY>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -337,6 +339,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
   static_assert(TY < 32, "the own-row mask holds one bit per tile row");
   using BX = TmaBox64<TX, TY>;
   static_assert(!TMA || (sizeof(R) == 8 && BX::FITS), "FP64 boxes in the face-flux arrays");
+  static_assert(!TAPE || (sizeof(R) == 8 && !TMA), "the tape is FP64 and recorded by the plain loads");
   __shared__ __align__(8) uint64_t s_bar;   // TMA completion
   __shared__ unsigned s_phase;              // parity of the mbarrier phase the next box completes
 
@@ -486,6 +489,19 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
         sP[4 * G::NP + p] = pr.Bx;
         sP[5 * G::NP + p] = pr.By;
         nan_tile |= not_finite_p(pr.P);
+        if constexpr (TAPE) {
+          const int ox = qx - 2, oy = qy - 2;
+          if (ox >= 0 && ox < TX && oy >= 0 && oy < TY && i0 + ox < nx && j0 + oy < ny) {
+            const TapeOut& t = *a.tape;
+            t.P[0][idx] = pr.rho;
+            t.P[1][idx] = pr.vx;
+            t.P[2][idx] = pr.vy;
+            t.P[3][idx] = pr.P;
+            t.P[4][idx] = pr.Bx;
+            t.P[5][idx] = pr.By;
+            if (not_finite_p(pr.P)) *t.nan_seen = 1;
+          }
+        }
       }
     }
     if (!from_box) nan_tile = __syncthreads_or(nan_tile);   // (the box path ended with its own barrier)
@@ -654,7 +670,9 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
     const R inv_dx = R(g.inv_dx), inv_dy = R(g.inv_dy);
     const int bx_lo = (STAGE == 3 && (i0 > 0 || px)) ? -1 : 0;   // halo face column for the epilogue
     const int by_lo = (STAGE == 3 && (j0 > 0 || py)) ? -1 : 0;
-    for (int e = tid; e < G::NBX + G::NBY; e += NT) {
+    // (a taped stage 3 is run for what its floors change: it writes no state)
+    constexpr bool WRITE = !(TAPE && STAGE == 3);
+    for (int e = WRITE ? tid : G::NBX + G::NBY; e < G::NBX + G::NBY; e += NT) {
       const bool isy = e >= G::NBX;
       const int ee = isy ? e - G::NBX : e;
       int li, lj;
@@ -720,7 +738,19 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
       const R cr = sP[0 * G::NP + pc], cu = sP[1 * G::NP + pc], cv = sP[2 * G::NP + pc];
       const R cP = sP[3 * G::NP + pc], cBx = sP[4 * G::NP + pc], cBy = sP[5 * G::NP + pc];
       // apply_conserved_floors with the stage's (pre-CT) cell B (src/main.f90:113)
-      floor_hits += conserved_floors<R>(U[0], U[1], U[2], U[3], cBx, cBy, gamma, vol) ? 1u : 0u;
+      R W[4];   // TAPE: what goes into the floors
+      if constexpr (TAPE) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) W[q] = U[q];
+      }
+      const int hit1 = conserved_floors<R>(U[0], U[1], U[2], U[3], cBx, cBy, gamma, vol);
+      floor_hits += hit1 ? 1u : 0u;
+      if constexpr (TAPE) {
+        if (hit1) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) a.tape->Upre[q][idx] = W[q];
+        }
+      }
       // outflow boundary flux correction (src/main.f90:118-148)
       if (!px && i == 0) {
         const R hb = R(0.5) * (cBx * cBx + cBy * cBy);
@@ -747,12 +777,28 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) U[q] = R(1.0 / 3.0) * u0[q][idx] + R(2.0 / 3.0) * U[q];
       }
-      if (STAGE >= 2) floor_hits += conserved_floors<R>(U[0], U[1], U[2], U[3], cBx, cBy, gamma, vol) ? 1u : 0u;
+      int hit2 = 0;
+      if (STAGE >= 2) {
+        if constexpr (TAPE) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) out[q][idx] = U[q];
+          for (int q = 0; q < 4; ++q) W[q] = U[q];
+        }
+        hit2 = conserved_floors<R>(U[0], U[1], U[2], U[3], cBx, cBy, gamma, vol);
+        floor_hits += hit2 ? 1u : 0u;
+      }
+      if constexpr (TAPE) {
+        if (hit2) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) a.tape->Ublend[q][idx] = W[q];
+        }
+        a.tape->hit[idx] = (unsigned char)((hit1 ? 1 : 0) | (hit2 ? 2 : 0));
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (WRITE) out[q][idx] = U[q];
       const R bxn = (STAGE == 3) ? sBx[lj * G::BXW + (li + 1)] : R(0);
       const R byn = (STAGE == 3) ? sBy[(lj + 1) * G::BYW + li] : R(0);
-      if (STAGE == 3) {   // (stages 1, 2 stored the new face B in phase 3a)
+      if (STAGE == 3 && WRITE) {   // (stages 1, 2 stored the new face B in phase 3a)
         out[4][idx] = bxn;
         out[5][idx] = byn;
       }
@@ -760,7 +806,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
       // epilogue: primitives of U^{n+1} (next step's CFL, src/main.f90:69-79),
       // div B (src/main.f90:276), |B| and totals -- over the grid's own rows (a
       // y-slab's ghost rows are left out)
-      if (STAGE == 3 && ((s_own >> lj) & 1u)) {
+      if (STAGE == 3 && WRITE && ((s_own >> lj) & 1u)) {
         const R bxm = sBx[lj * G::BXW + li];
         const R bym = sBy[lj * G::BYW + li];
         const bool hx = (i > 0) || px, hy = (j > 0) || py;
