@@ -53,6 +53,7 @@
 #include "chimera_types.h"
 #include "dual.cuh"
 #include "face_vjp.cuh"
+#include "grid_dep.cuh"
 #include "kernel_table.h"
 #include "mhd_device.cuh"
 
@@ -260,6 +261,8 @@ __global__ void __launch_bounds__(128, SOLVER == RIEMANN_HLLD ? 4 : 5) k_rev_fac
   const int d = ydir ? 1 : 0;
   const int nx = g.nx, ny = g.ny;
   const long long n = (long long)nx * ny;
+  grid_wait();
+  grid_release();
   const bool full_bounds = *a.tape.nan_seen != 0;   // a NaN somewhere: the bounds' comparisons decide
   for (long long cc = blockIdx.x * (long long)blockDim.x + threadIdx.x; cc < n; cc += (long long)gridDim.x * blockDim.x) {
     const int c = int(cc);
@@ -444,6 +447,8 @@ __global__ void __launch_bounds__(RC_NT, 2) k_rev_cells(const __grid_constant__ 
   const unsigned n = unsigned(nx) * unsigned(ny);
   const int tiles_x = (nx + RC_TX - 1) / RC_TX, tiles_y = (ny + RC_TY - 1) / RC_TY;
   const int tid = threadIdx.x;
+  grid_wait();
+  grid_release();
   for (int tile = blockIdx.x; tile < tiles_x * tiles_y; tile += gridDim.x) {
     const int i0 = (tile % tiles_x) * RC_TX, j0 = (tile / tiles_x) * RC_TY;
     // this thread's slopes: the cell, its neighbours in the slope (each side's ghost
@@ -517,17 +522,17 @@ __global__ void __launch_bounds__(RC_NT, 2) k_rev_cells(const __grid_constant__ 
 #pragma unroll
       for (int w = 0; w < 2; ++w) {
         if (!have) break;
-        const int q = q0 + w;
         const double* const wl = sw[(q0 >> 1) & 1][w][0];
         const double* const wr = sw[(q0 >> 1) & 1][w][1];
+        const int q = q0 + w;
         // this cell is the low cell of faces (c, x) and (c, y), the high cell of (fxm, x) and (fym, y)
         double v = a.fL[0][q][c] + a.fL[1][q][c];
-        if (resetx) v += a.fX[0][q][c];
-        if (resety) v += a.fX[1][q][c];
         if (fxm >= 0) v += a.fR[0][q][fxm];
         if (fym >= 0) v += a.fR[1][q][fym];
         if (ex) v += a.fR[0][q][c];
         if (ey) v += a.fR[1][q][c];
+        if (resetx) v += a.fX[0][q][c];
+        if (resety) v += a.fX[1][q][c];
         // slopes: s(p) uses f(p-1), f(p), f(p+1).  The cell's own slope, with its own
         // ghost below / above where that side is outflow, then the slopes of the cells
         // whose low / high neighbour it is (across a periodic side, through the wrap)
@@ -804,6 +809,23 @@ extern "C" void chimera_adjoint_destroy(chimera_adjoint* a) {
   delete a;
 }
 
+// A launch that overlaps the end of the kernel before it in the stream (grid_wait in
+// the kernels).
+static cudaError_t launch_after(const void* fn, dim3 grid, int threads, size_t smem, cudaStream_t stream, void** args,
+                                bool overlap = true) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 // The three stages from U_n on the stage kernels ks.  Taped: U1 and U2 stay in the
 // handle's buffers and U_{n+1} is not written.  Else U_{n+1} goes to out, which
 // serves as U1 on the way.  Control is the same for all three: dry launches leave
@@ -840,24 +862,13 @@ static int run_stages(chimera_adjoint* a, const KernelSet& ks, const int* grid, 
     const KernelEntry& e = ks.stage[a->g.riemann - 1][k];
     s.tape = taped ? &a->desc->tape[k] : nullptr;
     void* args[] = {&s};
-    // a stage's launch overlaps the end of the one before it (grid_wait in the kernels)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid[k]);
-    cfg.blockDim = dim3(e.nt);
-    cfg.dynamicSmemBytes = e.smem;
-    cfg.stream = a->stream;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = k > 0 ? 1 : 0;
-    if (cudaLaunchKernelExC(&cfg, e.fn, args) != cudaSuccess) return adj_fail();
+    if (launch_after(e.fn, dim3(grid[k]), e.nt, e.smem, a->stream, args, k > 0) != cudaSuccess) return adj_fail();
   }
   return CHIMERA_OK;
 }
 
 // One stage of the reverse sweep from input U and output adjoint lout to lin.
-static void rev_stage(chimera_adjoint* a, int stage, double dt, const double* const* U, const double* const* lout,
+static int rev_stage(chimera_adjoint* a, int stage, double dt, const double* const* U, const double* const* lout,
                       double* const* lin) {
   RevStage r;
   r.g = a->g;
@@ -879,13 +890,16 @@ static void rev_stage(chimera_adjoint* a, int stage, double dt, const double* co
   }
   for (int d = 0; d < 2; ++d) r.fflag[d] = a->fflag[d];
   const dim3 faces(unsigned(std::min<long long>((a->n + 127) / 128, 1 << 20)), 2);
-  switch (a->g.riemann) {
-    case CHIMERA_RIEMANN_RUSANOV: k_rev_faces<RIEMANN_RUSANOV><<<faces, 128, 0, a->stream>>>(r); break;
-    case CHIMERA_RIEMANN_HLLE: k_rev_faces<RIEMANN_HLLE><<<faces, 128, 0, a->stream>>>(r); break;
-    default: k_rev_faces<RIEMANN_HLLD><<<faces, 128, 0, a->stream>>>(r); break;
-  }
+  const void* fn = (a->g.riemann == CHIMERA_RIEMANN_RUSANOV) ? (const void*)&k_rev_faces<RIEMANN_RUSANOV>
+                   : (a->g.riemann == CHIMERA_RIEMANN_HLLE)  ? (const void*)&k_rev_faces<RIEMANN_HLLE>
+                                                             : (const void*)&k_rev_faces<RIEMANN_HLLD>;
+  void* args[] = {&r};
+  if (launch_after(fn, faces, 128, 0, a->stream, args) != cudaSuccess) return adj_fail();
   const long long tiles = (long long)((a->g.nx + RC_TX - 1) / RC_TX) * ((a->g.ny + RC_TY - 1) / RC_TY);
-  k_rev_cells<<<unsigned(std::min<long long>(tiles, 1 << 20)), RC_NT, 0, a->stream>>>(r);
+  if (launch_after((const void*)&k_rev_cells, dim3(unsigned(std::min<long long>(tiles, 1 << 20))), RC_NT, 0, a->stream,
+                   args) != cudaSuccess)
+    return adj_fail();
+  return CHIMERA_OK;
 }
 
 // Whether any of the six output arrays overlaps one of the six inputs.
@@ -916,9 +930,9 @@ extern "C" int chimera_adjoint_step(chimera_adjoint* a, const double* const* U_n
   // lambda_n may be U_n's memory: the last stage reads U_n around the cells it writes
   const bool aside = overlaps(a, U_n, lambda_n);
   double* const* dst = aside ? a->lA : lambda_n;
-  rev_stage(a, 3, dt, a->U2, lambda_next, a->lA);   // lambda_U2 -> lA
-  rev_stage(a, 2, dt, a->U1, a->lA, a->lB);         // lambda_U1 -> lB
-  rev_stage(a, 1, dt, U_n, a->lB, dst);             // lambda_Un, with the blends' share
+  if ((rc = rev_stage(a, 3, dt, a->U2, lambda_next, a->lA))) return rc;   // lambda_U2 -> lA
+  if ((rc = rev_stage(a, 2, dt, a->U1, a->lA, a->lB))) return rc;         // lambda_U1 -> lB
+  if ((rc = rev_stage(a, 1, dt, U_n, a->lB, dst))) return rc;             // lambda_Un, with the blends' share
   if (aside && (rc = copy6(a, lambda_n, a->lA))) return rc;
   if (cudaGetLastError() != cudaSuccess) return CHIMERA_ERR_CUDA;
   if (cudaStreamSynchronize(a->stream) != cudaSuccess) return adj_fail();

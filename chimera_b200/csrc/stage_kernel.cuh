@@ -22,6 +22,7 @@
 #pragma once
 #include "mhd_device.cuh"
 #include "chimera_types.h"
+#include "grid_dep.cuh"
 #include "tma.cuh"
 
 namespace chimera {
@@ -63,15 +64,6 @@ __device__ __forceinline__ int map_index(int g, int n, int plo, int phi) {
   }
   return g < 0 ? 0 : n - 1;
 }
-
-// Programmatic dependent launch: the host lets a stage kernel start while the
-// one before it in the stream still runs.  grid_wait() holds until that one has
-// completed, its writes visible; everything a kernel reads comes after it.
-// grid_release(), once every CTA of a grid has called it or ended, lets the next
-// kernel's CTAs take up free places and wait there.  Both do nothing in an
-// ordinary launch.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename R> struct StageTileSmem;
 
