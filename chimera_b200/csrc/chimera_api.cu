@@ -41,6 +41,48 @@ __global__ void k_f32_to_f64(const float* __restrict__ src, double* __restrict__
     dst[k] = double(src[k]);
 }
 
+// ---- whole states between a member's buffers and device arrays ----------------
+// The six fields of buffer set `which` (0: the state, in the set the device-side
+// parity names; 1: the other of the two; 2: U2) from or to pitched float64 arrays,
+// converted to the storage type T on the way; the parity is read on the device, so
+// that the host need not wait for the steps before.  Bound by HBM.
+struct FieldPtrs { double* p[6]; };
+template <typename T, bool IN>
+__global__ void __launch_bounds__(256) move_state_kernel(const Member* __restrict__ g, const Control* __restrict__ ctl,
+                                                         int which, FieldPtrs f, int ld) {
+  const int b = (which == 0) ? ctl->parity : (which == 1 ? 1 - ctl->parity : 2);
+  const int q = blockIdx.y;
+  T* __restrict__ st = static_cast<T*>(g->buf[b][q]);
+  double* __restrict__ ar = f.p[q];
+  const unsigned nx = unsigned(g->nx), n = nx * unsigned(g->ny), stride = gridDim.x * blockDim.x;   // n <= 2^31
+  for (unsigned k0 = blockIdx.x * blockDim.x + threadIdx.x; k0 < n; k0 += 4u * stride) {
+    double v[4];
+#pragma unroll
+    for (unsigned u = 0; u < 4; ++u) {   // four loads in flight
+      const unsigned k = k0 + u * stride;
+      if (k >= n || k < k0) continue;
+      const size_t at = (unsigned(ld) == nx) ? k : size_t(k / nx) * unsigned(ld) + k % nx;
+      v[u] = IN ? ar[at] : double(st[k]);
+    }
+#pragma unroll
+    for (unsigned u = 0; u < 4; ++u) {
+      const unsigned k = k0 + u * stride;
+      if (k >= n || k < k0) continue;
+      const size_t at = (unsigned(ld) == nx) ? k : size_t(k / nx) * unsigned(ld) + k % nx;
+      if (IN) st[k] = T(v[u]);
+      else ar[at] = v[u];
+    }
+    if (k0 + 4u * stride < k0) break;   // past 2^32
+  }
+}
+
+// t and output_count of a member; it is active while t < t_end.
+__global__ void set_time_kernel(Control* c, double t, int output_count, int active) {
+  c->t = t;
+  c->output_count = output_count;
+  c->active = active;
+}
+
 bool valid_bc(int b) { return b >= CHIMERA_BC_PERIODIC && b <= CHIMERA_BC_INFLOW; }
 
 // NVTX range over the host-side span of an API call or a kernel launch: named
@@ -373,6 +415,42 @@ static int run_steps(chimera_handle* h, int nsteps) {
 }
 
 static size_t cells_of(const chimera_cfg& c) { return size_t(c.nx) * size_t(c.ny); }
+
+// Whether the six arrays can be moved by a kernel: float64-aligned memory of the
+// handle's device, and no capture under way (the calls wait for the device, which a
+// capture refuses, as it always has).
+static bool movable(chimera_handle* h, const void* const* ptrs, int where) {
+  if (where != CHIMERA_DEVICE) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  for (int q = 0; q < 6; ++q) {
+    cudaPointerAttributes a;
+    if (reinterpret_cast<uintptr_t>(ptrs[q]) % sizeof(double) != 0 ||
+        cudaPointerGetAttributes(&a, ptrs[q]) != cudaSuccess || a.type != cudaMemoryTypeDevice ||
+        a.device != h->device) {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  return true;
+}
+
+template <bool IN>
+static int move_state(chimera_handle* h, int m, int which, const void* const* ptrs, int ld) {
+  FieldPtrs f;
+  for (int q = 0; q < 6; ++q) f.p[q] = static_cast<double*>(const_cast<void*>(ptrs[q]));
+  const size_t n = cells_of(h->cfg[m]);
+  const dim3 grid(unsigned(std::min<size_t>((n + 1023) / 1024, size_t(h->num_sms) * 8)), 6);
+  if (h->ks.elem_bytes == 8)
+    move_state_kernel<double, IN><<<grid, 256, 0, h->stream>>>(h->d_members + m, h->d_ctl + m, which, f, ld);
+  else
+    move_state_kernel<float, IN><<<grid, 256, 0, h->stream>>>(h->d_members + m, h->d_ctl + m, which, f, ld);
+  CK(cudaGetLastError());
+  return CHIMERA_OK;
+}
 
 static int tiles_for(const chimera_handle* h, int tx, int ty) {
   int t = 0;
@@ -743,6 +821,12 @@ int chimera_batch_set_state(chimera_handle* h, int m, const double* Mass, const 
   const void* ptrs[6] = {Mass, Momx, Momy, Energy, b_x, b_y};
   int rc = check_io(h, m, ptrs, ld, where);
   if (rc) return rc;
+  if (movable(h, ptrs, where)) {
+    // one kernel, once the work before it is done: the arrays are read right away
+    CK(cudaStreamSynchronize(h->stream));
+    h->dt_valid[m] = false;
+    return move_state<true>(h, m, 0, ptrs, ld);
+  }
   Control c;
   rc = read_ctl(h, m, &c);
   if (rc) return rc;
@@ -768,6 +852,12 @@ static int get_buffer(chimera_handle* h, int m, int which, double* const* ptrs, 
   int rc = check_io(h, m, p6, ld, where);
   if (rc) return rc;
   Control c;
+  if (movable(h, p6, where)) {   // one kernel and one wait
+    rc = move_state<false>(h, m, which, p6, ld);
+    if (!rc) rc = read_ctl(h, m, &c);
+    if (rc) return rc;
+    return c.status ? CHIMERA_ERR_NONFINITE : CHIMERA_OK;
+  }
   rc = read_ctl(h, m, &c);
   if (rc) return rc;
   const int b = (which == 0) ? c.parity : (which == 1 ? 1 - c.parity : 2);
@@ -935,14 +1025,11 @@ int chimera_step_host(chimera_handle* h, const double* const* in, double* const*
 
 int chimera_batch_set_time(chimera_handle* h, int m, double t, int output_count) {
   if (!h || m < 0 || m >= h->n || output_count < 1) return CHIMERA_ERR_BAD_ARG;
-  Control c;
-  int rc = read_ctl(h, m, &c);
-  if (rc) return rc;
-  c.t = t;
-  c.output_count = output_count;
-  c.active = (t < h->cfg[m].t_end) ? 1 : 0;
-  CK(cudaMemcpyAsync(h->d_ctl + m, &c, sizeof(Control), cudaMemcpyHostToDevice, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(h->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return CHIMERA_ERR_CUDA;   // dt_valid is the host's: not for a replay
+  set_time_kernel<<<1, 1, 0, h->stream>>>(h->d_ctl + m, t, output_count, (t < h->cfg[m].t_end) ? 1 : 0);
+  CK(cudaGetLastError());
   h->dt_valid[m] = false;
   return CHIMERA_OK;
 }

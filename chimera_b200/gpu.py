@@ -203,13 +203,24 @@ class Solver:
     def stream(self) -> int:
         return lib().chimera_stream(self._h) or 0
 
+    def _after_torch(self, arrays):
+        """Order the solver's stream after torch's current one, where CUDA tensors
+        may still be written or read."""
+        if not getattr(arrays[0], "is_cuda", False):
+            return
+        import torch
+        cur = torch.cuda.current_stream()
+        if cur.cuda_stream != self.stream and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.ExternalStream(self.stream).wait_stream(cur)
+
     def set_state(self, arrays: Sequence, member: int = 0):
         """Six conserved fields (Mass, Momx, Momy, Energy, b_x, b_y) of member
         ``member`` in: numpy arrays or CPU tensors are read completely before
         the call returns (page-locked ones included); CUDA tensors are copied
-        in order on the solver's stream."""
+        in order on the solver's stream, after torch's current stream."""
         c = self.cfgs[member]
         p, ld, where, keep = _ptrs(arrays, c.nx, c.ny)
+        self._after_torch(arrays)
         _check(lib().chimera_batch_set_state(self._h, member, *p, ld, where), "set_state")
 
     def get_state(self, member: int = 0, out=None, check: bool = True):
@@ -217,6 +228,7 @@ class Solver:
         if out is None:
             out = [np.empty((c.ny, c.nx), dtype=np.float64) for _ in range(6)]
         p, ld, where, keep = _ptrs(out, c.nx, c.ny, out=True)
+        self._after_torch(out)
         rc = lib().chimera_batch_get_state(self._h, member, *p, ld, where)
         if check:
             _check(rc, "get_state")
