@@ -246,6 +246,11 @@ static void harvest_profile(chimera_handle* h) {
 static int launch_raw(chimera_handle* h, const KernelEntry& k, int grid, int w_begin, int w_end,
                       cudaStream_t stream = nullptr, bool overlap = false);
 
+// The function an entry stands for on this handle.
+static const void* kernel_of(const chimera_handle* h, const KernelEntry& k) {
+  return (h->n == 1 && k.one) ? k.one : k.fn;
+}
+
 // kind: 0 = CFL kernel, 1..3 = stage kernels.  Stage kernels overlap their launch
 // with the end of the kernel before them (launch_raw).
 static int launch(chimera_handle* h, const KernelEntry& k, int grid, int kind) {
@@ -286,6 +291,7 @@ static int launch_raw(chimera_handle* h, const KernelEntry& k, int grid, int w_b
   a.counters = h->counters;
   a.dry = h->dry;
   a.tape = nullptr;
+  a.one = h->hm[0];
   void* args[] = {&a};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
@@ -297,14 +303,14 @@ static int launch_raw(chimera_handle* h, const KernelEntry& k, int grid, int w_b
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  CK(cudaLaunchKernelExC(&cfg, k.fn, args));
+  CK(cudaLaunchKernelExC(&cfg, kernel_of(h, k), args));
   return CHIMERA_OK;
 }
 
 // CTAs of kernel k that the device holds at once.
 static int resident_ctas(const chimera_handle* h, const KernelEntry& k) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.nt, k.smem) != cudaSuccess || per_sm < 1)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel_of(h, k), k.nt, k.smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   cudaGetLastError();
   return per_sm * h->num_sms;
@@ -526,8 +532,13 @@ static std::vector<int> small_variants(const chimera_handle* h) {
 // tiles, 39 on 16 x 8, 43 on 16 x 16, 66 on 32 x 16; 192^2 50, 42, 43, 68;
 // 256^2 85, 70, 52, 67, of which the device holds all 16 x 16 tiles but only
 // 296 of the 8 x 8 and 16 x 8 ones; rotor 320^2 125, 103, 83, 83).
-// Larger grids, FP64: variant 0, 32 x 16 tiles with TMA loads (rotor 1024^2
-// HLLE 509 us a step, the next best 550).  FP32-bulk: variant 9, the same tile at three CTAs
+// Larger grids, FP64, one grid: variant 10, 32 x 15 tiles of 384 threads, 24 warps an
+// SM (rotor 1024^2 HLLE 462 us a step, 487 on the 32 x 16 tile of 256 threads, both
+// with the descriptor in the launch; Rusanov 2048^2 1.69 ms against 1.77), and for
+// HLLD variant 11, one CTA of 768 threads an SM, whose warps share the longer code's
+// instruction cache (Kelvin-Helmholtz 2048^2 2.69 ms; two CTAs of 384 2.91, of 256
+// 2.96).  FP64 batches: variant 0, whose kernels spill less with the descriptor in
+// memory.  FP32-bulk: variant 9, the 32 x 16 tile at three CTAs
 // an SM with TMA loads, the fastest for every solver (Kelvin-Helmholtz 4096^2
 // HLLD 4.84 ms a step against variant 0's 5.50, 2048^2 Rusanov 0.970 against
 // 1.134, rotor 1024^2 HLLE 280 us against 292).  FP32 on FP64 storage: variant
@@ -542,7 +553,8 @@ static int default_variant(const chimera_handle* h) {
   }
   if (h->precision == CHIMERA_FP32_BULK) return 9;
   if (h->precision == CHIMERA_FP32_MIXED) return h->riemann == CHIMERA_RIEMANN_HLLD ? 0 : 1;
-  return 0;
+  if (h->n > 1) return 0;
+  return h->riemann == CHIMERA_RIEMANN_HLLD ? 11 : 10;
 }
 
 extern "C" {
@@ -608,7 +620,7 @@ int chimera_batch_create(int n_members, const chimera_cfg* cfgs, void* stream, c
     else fp32m_kernels(v, &h->variants[v]);
     for (int r = 0; r < 3; ++r)
       for (int st = 0; st < 3; ++st)
-        cudaFuncSetAttribute(h->variants[v].stage[r][st].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(kernel_of(h, h->variants[v].stage[r][st]), cudaFuncAttributeMaxDynamicSharedMemorySize,
                              int(h->variants[v].stage[r][st].smem));
   }
   cudaGetLastError();
@@ -1265,6 +1277,7 @@ int chimera_slab_ghost_rows(chimera_handle* h, int ghost_lo, int ghost_hi) {
   if (ghost_lo + ghost_hi >= h->cfg[0].ny) return CHIMERA_ERR_BAD_ARG;
   h->hm[0].skip_lo = ghost_lo;
   h->hm[0].skip_hi = ghost_hi;
+  drop_graph(h);   // its launches carry the descriptor
   CK(cudaMemcpyAsync(h->d_members, h->hm.data(), sizeof(Member) * h->n, cudaMemcpyHostToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   h->dt_valid[0] = false;

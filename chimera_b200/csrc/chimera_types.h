@@ -89,6 +89,7 @@ struct StageArgs {
   int counters;            // count MOOD resets / floor hits
   int dry;                 // timing run: write scratch only, leave Control untouched
   const TapeOut* tape;     // TAPE kernels only
+  Member one;              // ONE kernels (a single grid): its descriptor
 };
 
 }  // namespace chimera

@@ -10,6 +10,7 @@ struct KernelEntry {
   size_t smem;         // dynamic shared memory bytes
   int tx, ty, nt;      // tile shape and block size
   int box_w = 0, box_h = 0;   // TMA box of the stage input (elements), 0 = plain loads
+  const void* one = nullptr;  // the instantiation for a single grid (ONE), if there is one
 };
 
 struct KernelSet {
@@ -21,6 +22,7 @@ struct KernelSet {
 // Tile-shape variants per precision (for the autotuner).
 int fp64_variant_count();
 void fp64_kernels(int variant, KernelSet* out);
+void fp64_one_kernels(int variant, KernelSet* ks);   // (called by fp64_kernels)
 void fp64_mixed_pair_kernels(KernelSet* out);
 // The FP64 stage kernels that record the adjoint's tape (no CFL kernel).
 void tape_kernels(bool small, KernelSet* out);

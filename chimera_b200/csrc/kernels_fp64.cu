@@ -25,9 +25,9 @@ void fill(KernelSet* ks) {
 }
 }  // namespace
 
-// Tile shapes and occupancy targets the autotuner chooses from; the default
-// (variant 0) loads the stage input of interior tiles by TMA.
-int fp64_variant_count() { return 10; }
+// Tile shapes and occupancy targets the autotuner chooses from.  Variants 0, 10 and
+// 11 load the stage input of interior tiles by TMA.
+int fp64_variant_count() { return 12; }
 
 void fp64_kernels(int variant, KernelSet* out) {
   switch (variant) {
@@ -43,8 +43,13 @@ void fp64_kernels(int variant, KernelSet* out) {
     case 7: fill<8, 8, 192, 2>(out); break;
     case 8: fill<16, 8, 192, 2>(out); break;
     case 9: fill<16, 16, 320, 2>(out); break;
+    // 24 warps an SM, for single grids: three passes over the faces (1105 on 384
+    // threads, 2292 on 768)
+    case 10: fill<32, 15, 384, 2, false, true>(out); break;
+    case 11: fill<64, 16, 768, 1, false, true>(out); break;
     default: fill<32, 16, 256, 2, false, true>(out); break;   // phase 1 from TMA boxes (interior tiles)
   }
+  fp64_one_kernels(variant, out);
 }
 
 // The one tile for grids with a periodic side facing a non-periodic one.

@@ -439,15 +439,14 @@ __device__ __forceinline__ Flux5<R> hlld(R gamma, R rhoL, R rhoR, R vxL, R vxR, 
   return hlld_guard(F, SL, SR, FL, FR, rhoL, rhoR, vxL, vxR, vyL, vyR, enL, enR, ByL, ByR, dM, dMn, dMt, dE, dB);
 }
 
-// rcp_gm1: RN(1/(gamma - 1)) for div_by, or 0.  HLLE keeps IEEE division: with
-// div_by its FP64 stage-3 kernel spilled 32 / 84 bytes per thread instead of
-// 20 / 36 and ran 0.1% slower on the rotor; Rusanov and HLLD gain.
+// rcp_gm1: RN(1/(gamma - 1)) for div_by, or 0.
 template <typename R, int SOLVER>
 __device__ __forceinline__ Flux5<R> riemann(R gamma, R rL, R rR, R uL, R uR, R vL, R vR, R PL, R PR,
                                             R BnL, R BnR, R BtL, R BtR, double rcp_gm1 = 0.0) {
   if (SOLVER == RIEMANN_RUSANOV)
     return rusanov<R>(gamma, rL, rR, uL, uR, vL, vR, PL, PR, BnL, BnR, BtL, BtR, rcp_gm1);
-  if (SOLVER == RIEMANN_HLLE) return hlle<R>(gamma, rL, rR, uL, uR, vL, vR, PL, PR, BnL, BnR, BtL, BtR);
+  if (SOLVER == RIEMANN_HLLE)
+    return hlle<R>(gamma, rL, rR, uL, uR, vL, vR, PL, PR, BnL, BnR, BtL, BtR, rcp_gm1);
   return hlld<R>(gamma, rL, rR, uL, uR, vL, vR, PL, PR, BnL, BnR, BtL, BtR, rcp_gm1);
 }
 

@@ -48,6 +48,12 @@ __device__ __forceinline__ void* load_ptr(void* const* p) {
   return reinterpret_cast<void*>(v);
 }
 
+// The descriptor of member m; ONE: of the launch's single grid.
+template <bool ONE> __device__ __forceinline__ const Member& member_of(const StageArgs& a, int m) {
+  if constexpr (ONE) return a.one;
+  else return a.members[m];
+}
+
 // Source cell of a (possibly out-of-domain) tile position: periodic wrap or
 // the nearest cell, by the rule of the side it lies beyond (plo below 0, phi
 // at n and above; src/mhd_bc.f90:36-121 takes each side on its own).
@@ -313,10 +319,14 @@ __device__ void member_finish(const Member& g, Control* ctl, const double* part,
 // a mixed pair run the MIXBC = false instantiations.
 // TAPE: the adjoint's forward re-run; the stage's primitives and what its floors
 // changed are recorded (TapeOut); stage 3 writes nothing else.
+// ONE: a single grid, whose descriptor comes with the launch.  Its constants and
+// pointers are then operands in the constant bank instead of registers held (or
+// spilled) through phase 2: HLLE's stage 3 needs 80 registers with 12 bytes of
+// spills where it needed 128 with 36, so that 24 warps run on an SM for 16.
 // ----------------------------------------------------------------------------
 template <typename R, int SOLVER, int STAGE, int TX, int TY, int NT, int MINB, bool KEEP_IN = false,
-          bool TMA = false, int UNIT = UNIT_FP64, bool MIXBC = false, bool TAPE = false>
-__global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
+          bool TMA = false, int UNIT = UNIT_FP64, bool MIXBC = false, bool TAPE = false, bool ONE = false>
+__global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__ StageArgs a) {
   using G = TileGeom<TX, TY>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* sP = reinterpret_cast<R*>(smem_raw);
@@ -350,8 +360,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
   grid_wait();
 
   for (int w = a.work_begin + blockIdx.x; w < a.total_tiles; w += gridDim.x) {
-    const int m = (a.n_members == 1) ? 0 : a.tile_member[w];
-    const Member& g = a.members[m];
+    const int m = (ONE || a.n_members == 1) ? 0 : a.tile_member[w];
+    const Member& g = member_of<ONE>(a, m);
     Control* ctl = a.ctl + m;
     if (ctl->active == 0) continue;  // uniform across the CTA
     const int nx = g.nx, ny = g.ny;
@@ -525,12 +535,20 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
         own_ym = !py && pyh && gay == ny;
         own_bm = ydir ? (!py && pyh && gay + 1 == ny) : (!px && pxh && gax + 1 == nx);
       }
+      // the low cell's value of slot q: rho, normal and tangential velocity, P,
+      // normal and tangential B (the fields 1, 2 and 4, 5 trade places for a y face:
+      // two base pointers in place of eight selected inputs)
+      const R* const cell_n = sP + pa + (ydir ? G::NP : 0);
+      const R* const cell_t = sP + pa - (ydir ? G::NP : 0);
+      auto field = [&](int q) -> const R* {
+        return ((q == 1 || q == 4) ? cell_n : (q == 2 || q == 5) ? cell_t : sP + pa) + q * G::NP;
+      };
       const bool own_np = ydir ? own_yp : own_xp;   // the high cell is the low cell's own ghost
 #pragma unroll
       for (int q = 0; q < 6; ++q) {
-        const R* s = sP + q * G::NP;
-        const R fm = s[pa - on], f0 = s[pa];
-        R fp = s[pa + on], fpp = s[pa + 2 * on];
+        const R* s = field(q);
+        const R fm = s[-on], f0 = s[0];
+        R fp = s[on], fpp = s[2 * on];
         if (MIXBC && own_np) { fp = f0; fpp = f0; }
         const R fb0 = (MIXBC && own_bm) ? fp : f0;    // the high cell's low neighbour
         // apply_slope_limiter (src/mhd_derivatives.f90:50-127) or compute_gradients (:15-47)
@@ -577,9 +595,9 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
           if (!nan_tile && !((outside >> q) & 1u)) continue;
-          const R* s = sP + q * G::NP;
-          const R f0 = s[pa];
-          R nxp = s[pa + 1], nxm = s[pa - 1], nyp = s[pa + G::PX], nym = s[pa - G::PX];
+          const R* s = field(q);
+          const R f0 = s[0];
+          R nxp = s[1], nxm = s[-1], nyp = s[G::PX], nym = s[-G::PX];
           if (MIXBC && own_xp) nxp = f0;
           if (MIXBC && own_xm) nxm = f0;
           if (MIXBC && own_yp) nyp = f0;
@@ -598,29 +616,27 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
       }
       // thermal_pressure_check (src/mhd_derivatives.f90:232-293): reset all six
       // fields of a face slot to the low cell's values.
-      if (L[3] - R(0.5) * (L[4] * L[4] + L[5] * L[5]) < K<R>::P_floor) {
+      const bool coldL = L[3] - R(0.5) * (L[4] * L[4] + L[5] * L[5]) < K<R>::P_floor;
+      const bool coldR = Rv[3] - R(0.5) * (Rv[4] * Rv[4] + Rv[5] * Rv[5]) < K<R>::P_floor;
+      if (coldL || coldR) {
 #pragma unroll
-        for (int q = 0; q < 6; ++q) L[q] = sP[q * G::NP + pa];
-      }
-      if (Rv[3] - R(0.5) * (Rv[4] * Rv[4] + Rv[5] * Rv[5]) < K<R>::P_floor) {
-#pragma unroll
-        for (int q = 0; q < 6; ++q) Rv[q] = sP[q * G::NP + pa];
+        for (int q = 0; q < 6; ++q) {
+          const R f0 = field(q)[0];
+          if (coldL) L[q] = f0;
+          if (coldR) Rv[q] = f0;
+        }
       }
       mood_resets += reset ? 1u : 0u;
       // compute_fluxes, rotated for y faces (src/main.f90:394-401)
-      const R unL = ydir ? L[2] : L[1], unR = ydir ? Rv[2] : Rv[1];
-      const R utL = ydir ? L[1] : L[2], utR = ydir ? Rv[1] : Rv[2];
-      const R bnL = ydir ? L[5] : L[4], bnR = ydir ? Rv[5] : Rv[4];
-      const R btL = ydir ? L[4] : L[5], btR = ydir ? Rv[4] : Rv[5];
-      Flux5<R> F = riemann<R, SOLVER>(gamma, L[0], Rv[0], unL, unR, utL, utR, L[3], Rv[3], bnL, bnR, btL, btR,
-                                      rcp_gm1);
-      R* dst = ydir ? sFy : sFx;
+      Flux5<R> F = riemann<R, SOLVER>(gamma, L[0], Rv[0], L[1], Rv[1], L[2], Rv[2], L[3], Rv[3], L[4], Rv[4], L[5],
+                                      Rv[5], rcp_gm1);
+      R* dst = (ydir ? sFy : sFx) + ff;
       const int NF = ydir ? G::NFY : G::NFX;
-      dst[0 * NF + ff] = F.mass;
-      dst[1 * NF + ff] = ydir ? F.momt : F.momn;   // x momentum flux
-      dst[2 * NF + ff] = ydir ? F.momn : F.momt;   // y momentum flux
-      dst[3 * NF + ff] = F.energy;
-      dst[4 * NF + ff] = F.bt;                     // By flux (x faces) / Bx flux (y faces)
+      dst[0] = F.mass;
+      dst[ydir ? 2 * G::NFY : G::NFX] = F.momn;    // x momentum flux at 1, y momentum flux at 2
+      dst[ydir ? G::NFY : 2 * G::NFX] = F.momt;
+      dst[3 * NF] = F.energy;
+      dst[4 * NF] = F.bt;                          // By flux (x faces) / Bx flux (y faces)
     }
     if (a.counters && !a.dry) {
       unsigned s = __reduce_add_sync(0xffffffffu, mood_resets);
@@ -636,9 +652,15 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(StageArgs a) {
     R* __restrict__ out[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      in[q] = static_cast<const R*>(load_ptr(&g.buf[in_buf][q]));
-      u0[q] = static_cast<const R*>(load_ptr(&g.buf[sbuf][q]));
-      out[q] = static_cast<R*>(load_ptr(&g.buf[out_buf][q]));
+      if constexpr (ONE) {
+        in[q] = static_cast<const R*>(g.buf[in_buf][q]);
+        u0[q] = static_cast<const R*>(g.buf[sbuf][q]);
+        out[q] = static_cast<R*>(g.buf[out_buf][q]);
+      } else {
+        in[q] = static_cast<const R*>(load_ptr(&g.buf[in_buf][q]));
+        u0[q] = static_cast<const R*>(load_ptr(&g.buf[sbuf][q]));
+        out[q] = static_cast<R*>(load_ptr(&g.buf[out_buf][q]));
+      }
     }
 
     // ---- phase 3a: constrained transport -> new face B ------------------------
