@@ -655,9 +655,12 @@ static int adj_fail() {
   return CHIMERA_ERR_CUDA;
 }
 
+// An adjoint is one grid: the single-grid instantiation where there is one.
+static const void* function_of(const KernelEntry& k) { return k.one ? k.one : k.fn; }
+
 static int resident_ctas(const chimera_adjoint* a, const KernelEntry& k) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.nt, k.smem) != cudaSuccess || per_sm < 1)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, function_of(k), k.nt, k.smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   cudaGetLastError();
   return per_sm * a->sms;
@@ -667,13 +670,13 @@ static int tiles_of(const chimera_adjoint* a, const KernelEntry& k) {
   return ((a->g.nx + k.tx - 1) / k.tx) * ((a->g.ny + k.ty - 1) / k.ty);
 }
 
-// The stage kernels of this grid: 8 x 8 tiles where the device holds all of them at
-// once, else 32 x 16, as the solver's handles choose them (their TMA tiles need
-// tensor maps of the caller's arrays; plain loads here).
+// The stage kernels of this grid, as the solver's handles choose them: a small-grid
+// tile where the device holds all of them at once, else a large one (without the
+// caller's arrays' tensor maps it takes plain loads everywhere).
 static void pick_kernels(chimera_adjoint* a, bool mixed) {
   auto allow = [&](KernelSet& ks) {
     for (int s = 0; s < 3; ++s)
-      cudaFuncSetAttribute(ks.stage[a->g.riemann - 1][s].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(function_of(ks.stage[a->g.riemann - 1][s]), cudaFuncAttributeMaxDynamicSharedMemorySize,
                            int(ks.stage[a->g.riemann - 1][s].smem));
     cudaGetLastError();
   };
@@ -700,7 +703,7 @@ static void pick_kernels(chimera_adjoint* a, bool mixed) {
       allow(a->forward);
       if ((found = fits(a->forward))) break;
     }
-    if (!found) fp64_kernels(1, &a->forward);
+    if (!found) fp64_kernels(a->g.riemann == CHIMERA_RIEMANN_HLLD ? 11 : 10, &a->forward);
     tape_kernels(true, &a->taped);
     allow(a->taped);
     if (!fits(a->taped)) tape_kernels(false, &a->taped);
@@ -858,11 +861,12 @@ static int run_stages(chimera_adjoint* a, const KernelSet& ks, const int* grid, 
   s.slope_limiting = a->g.slope;
   s.mood = a->g.mood;
   s.dry = 1;
+  s.one = d.member;
   for (int k = 0; k < 3; ++k) {
     const KernelEntry& e = ks.stage[a->g.riemann - 1][k];
     s.tape = taped ? &a->desc->tape[k] : nullptr;
     void* args[] = {&s};
-    if (launch_after(e.fn, dim3(grid[k]), e.nt, e.smem, a->stream, args, k > 0) != cudaSuccess) return adj_fail();
+    if (launch_after(function_of(e), dim3(grid[k]), e.nt, e.smem, a->stream, args, k > 0) != cudaSuccess) return adj_fail();
   }
   return CHIMERA_OK;
 }

@@ -532,13 +532,15 @@ static std::vector<int> small_variants(const chimera_handle* h) {
 // tiles, 39 on 16 x 8, 43 on 16 x 16, 66 on 32 x 16; 192^2 50, 42, 43, 68;
 // 256^2 85, 70, 52, 67, of which the device holds all 16 x 16 tiles but only
 // 296 of the 8 x 8 and 16 x 8 ones; rotor 320^2 125, 103, 83, 83).
-// Larger grids, FP64, one grid: variant 10, 32 x 15 tiles of 384 threads, 24 warps an
-// SM (rotor 1024^2 HLLE 462 us a step, 487 on the 32 x 16 tile of 256 threads, both
-// with the descriptor in the launch; Rusanov 2048^2 1.69 ms against 1.77), and for
-// HLLD variant 11, one CTA of 768 threads an SM, whose warps share the longer code's
-// instruction cache (Kelvin-Helmholtz 2048^2 2.69 ms; two CTAs of 384 2.91, of 256
-// 2.96).  FP64 batches: variant 0, whose kernels spill less with the descriptor in
-// memory.  FP32-bulk: variant 9, the 32 x 16 tile at three CTAs
+// Larger grids, FP64, one grid: 24 warps an SM, variant 10 (two CTAs of 384 threads,
+// 32 x 15 tiles) or 11 (one of 768, 64 x 16), whichever gives the fullest SM the
+// fewer cells; us a step: rotor 1024^2 HLLE 458 and 456 (32 x 16 tiles of 256 threads
+// 486), Rusanov 2048^2 1673 and 1650 (1762), HLLE 512^2 128 and 134 (142).  HLLD always
+// 11, whose warps share the longer code's instruction cache: Kelvin-Helmholtz 2048^2
+// 2.67 ms, 2.91 on 10, 2.95 on the 256 threads; 512^2 204, 212, 229 us.  FP64 batches:
+// the same 11 for HLLD (1484 us a step on a 32-member ensemble, 1543 on variant 0),
+// else variant 0 (Rusanov 994, 995 on 10; HLLE 1042, 1075), since they spill more at 80
+// registers.  FP32-bulk: variant 9, the 32 x 16 tile at three CTAs
 // an SM with TMA loads, the fastest for every solver (Kelvin-Helmholtz 4096^2
 // HLLD 4.84 ms a step against variant 0's 5.50, 2048^2 Rusanov 0.970 against
 // 1.134, rotor 1024^2 HLLE 280 us against 292).  FP32 on FP64 storage: variant
@@ -553,8 +555,14 @@ static int default_variant(const chimera_handle* h) {
   }
   if (h->precision == CHIMERA_FP32_BULK) return 9;
   if (h->precision == CHIMERA_FP32_MIXED) return h->riemann == CHIMERA_RIEMANN_HLLD ? 0 : 1;
+  if (h->riemann == CHIMERA_RIEMANN_HLLD) return 11;
   if (h->n > 1) return 0;
-  return h->riemann == CHIMERA_RIEMANN_HLLD ? 11 : 10;
+  auto fullest = [&](int v) {   // cells of the SM that gets the most tiles
+    const KernelEntry& k = h->variants[v].stage[h->riemann - 1][0];
+    const long long ctas = resident_ctas(h, k), waves = (tiles_for(h, k.tx, k.ty) + ctas - 1) / ctas;
+    return waves * (ctas / h->num_sms) * k.tx * k.ty;
+  };
+  return fullest(10) < fullest(11) ? 10 : 11;
 }
 
 extern "C" {

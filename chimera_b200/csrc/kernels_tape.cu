@@ -12,7 +12,7 @@ void fill(KernelSet* ks) {
   const size_t smem = TileGeom<TX, TY>::template smem_bytes<double>();
 #define CHIMERA_ENTRY(S, K) \
   ks->stage[S - 1][K - 1] = KernelEntry{                                                                  \
-      (const void*)&stage_kernel<double, S, K, TX, TY, NT, MINB, false, false, UNIT_TAPE, MIXBC, true>,    \
+      (const void*)&stage_kernel<double, S, K, TX, TY, NT, MINB, false, false, UNIT_TAPE, MIXBC, true, true>, \
                                         smem, TX, TY, NT}
   CHIMERA_ENTRY(1, 1); CHIMERA_ENTRY(1, 2); CHIMERA_ENTRY(1, 3);
   CHIMERA_ENTRY(2, 1); CHIMERA_ENTRY(2, 2); CHIMERA_ENTRY(2, 3);
@@ -24,7 +24,7 @@ void fill(KernelSet* ks) {
 }  // namespace
 
 // small: 8 x 8 tiles, for grids of which the device holds all of them at once
-void tape_kernels(bool small, KernelSet* out) { small ? fill<8, 8, 192, 2>(out) : fill<32, 16, 256, 2>(out); }
+void tape_kernels(bool small, KernelSet* out) { small ? fill<8, 8, 192, 2>(out) : fill<32, 15, 384, 2>(out); }
 void tape_mixed_pair_kernels(KernelSet* out) { fill<32, 16, 256, 2, true>(out); }
 
 }  // namespace chimera

@@ -48,10 +48,21 @@ __device__ __forceinline__ void* load_ptr(void* const* p) {
   return reinterpret_cast<void*>(v);
 }
 
-// The descriptor of member m; ONE: of the launch's single grid.
-template <bool ONE> __device__ __forceinline__ const Member& member_of(const StageArgs& a, int m) {
+// The descriptor of a tile's grid.  ONE: the launch's single grid's; else a copy in
+// shared memory, made at the tile's start.
+template <bool ONE> __device__ __forceinline__ const Member& descriptor(const StageArgs& a, const Member& s) {
   if constexpr (ONE) return a.one;
-  else return a.members[m];
+  else return s;
+}
+
+// A constant of the grid, read where it is used: an operand in the constant bank
+// (ONE), else from the shared copy by a load the compiler does not move, so that it
+// takes no register through the phases between.
+template <bool ONE> __device__ __forceinline__ double grid_const(const double& x) {
+  if constexpr (ONE) return x;
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(smem_addr(&x)));
+  return v;
 }
 
 // Source cell of a (possibly out-of-domain) tile position: periodic wrap or
@@ -323,6 +334,9 @@ __device__ void member_finish(const Member& g, Control* ctl, const double* part,
 // pointers are then operands in the constant bank instead of registers held (or
 // spilled) through phase 2: HLLE's stage 3 needs 80 registers with 12 bytes of
 // spills where it needed 128 with 36, so that 24 warps run on an SM for 16.
+// Batches copy the descriptor of each tile's grid to shared memory and read it there
+// phase by phase (32-member ensemble, us a step: Rusanov 1016 with the constants in
+// registers, 994 so; HLLE 1057, 1042; HLLD 1588, 1543).
 // ----------------------------------------------------------------------------
 template <typename R, int SOLVER, int STAGE, int TX, int TY, int NT, int MINB, bool KEEP_IN = false,
           bool TMA = false, int UNIT = UNIT_FP64, bool MIXBC = false, bool TAPE = false, bool ONE = false>
@@ -335,6 +349,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
   R* sBx = sFy + 5 * G::NFY;
   R* sBy = sBx + G::NBX;
   R* sU = sBy + G::NBY;            // KEEP_IN: [4][TX * TY] the stage input of the tile's own cells
+  __shared__ Member s_member;
   __shared__ double red[6 * (NT / 32)];
   __shared__ int s_last;
   __shared__ unsigned s_own;   // stage 3: bit r set if tile row r is one of the grid's own rows
@@ -361,9 +376,14 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
 
   for (int w = a.work_begin + blockIdx.x; w < a.total_tiles; w += gridDim.x) {
     const int m = (ONE || a.n_members == 1) ? 0 : a.tile_member[w];
-    const Member& g = member_of<ONE>(a, m);
     Control* ctl = a.ctl + m;
     if (ctl->active == 0) continue;  // uniform across the CTA
+    if constexpr (!ONE) {
+      for (int k = tid; k < int(sizeof(Member) / sizeof(int)); k += NT)
+        reinterpret_cast<int*>(&s_member)[k] = reinterpret_cast<const int*>(a.members + m)[k];
+      __syncthreads();
+    }
+    const Member& g = descriptor<ONE>(a, s_member);
     const int nx = g.nx, ny = g.ny;
     const int px = g.periodic_x, py = g.periodic_y;                   // low sides
     const int pxh = MIXBC ? g.periodic_xhi : px, pyh = MIXBC ? g.periodic_yhi : py;   // high sides
@@ -377,10 +397,6 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
       const int lo = min(max(g.skip_lo - j0, 0), TY), hi = min(max(ny - g.skip_hi - j0, 0), TY);
       s_own = ((1u << hi) - 1u) & ~((1u << lo) - 1u);
     }
-    const R gamma = R(g.gamma);
-    const R vol = R(g.vol);
-    const double rcp_vol = g.rcp_vol, rcp_gm1 = g.rcp_gm1;
-    const R dt = R(ctl->dt);
     const int sbuf = ctl->parity, obuf = 1 - sbuf;
     const int in_buf = (STAGE == 1) ? sbuf : (STAGE == 2 ? obuf : 2);
     const int out_buf = (STAGE == 2) ? 2 : obuf;
@@ -418,6 +434,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
           }
         }
         const bool ok = mbar_wait(&s_bar, s_phase, TMA_POLLS);
+        const R gamma = R(grid_const<ONE>(g.gamma)), vol = R(grid_const<ONE>(g.vol));
+        const double rcp_vol = grid_const<ONE>(g.rcp_vol);
         for (int p = tid; p < G::NP && ok; p += NT) {
           const int qx = p % G::PX, qy = p / G::PX;
           const int b = (qy + 1) * BX::BW + (qx + 2);   // box element of cell (i0-2+qx, j0-2+qy)
@@ -460,6 +478,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
       const R* __restrict__ in[6];
 #pragma unroll
       for (int q = 0; q < 6; ++q) in[q] = reinterpret_cast<const R*>(g.buf[in_buf][q]);
+      const R gamma = R(grid_const<ONE>(g.gamma)), vol = R(grid_const<ONE>(g.vol));
+      const double rcp_vol = grid_const<ONE>(g.rcp_vol);
       for (int p = tid; p < G::NP; p += NT) {
         const int qx = p % G::PX, qy = p / G::PX;
         const int si = map_index(i0 - 2 + qx, nx, px, pxh);
@@ -518,9 +538,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
       const int lj = ydir ? ff / G::FYW : ff / G::FXW;
       const int pa = (lj + 1) * G::PX + (li + 1);    // cell on the low side of the face
       const int on = ydir ? G::PX : 1;               // offset along the face normal
-      const R inv_h = R(ydir ? g.inv_dy : g.inv_dx);
-      const R inv_2h = R(ydir ? g.inv_2dy : g.inv_2dx);
-      const R hh = R(ydir ? g.hy : g.hx);             // 0.5 * spacing
+      const R inv_h = R(grid_const<ONE>(ydir ? g.inv_dy : g.inv_dx));
+      const R hh = R(grid_const<ONE>(ydir ? g.hy : g.hx));             // 0.5 * spacing
       R L[6], Rv[6];
       unsigned outside = 0;   // bit q: a state of field q is not between the low and the high cell's values
       // mixed pairs: the low cell's neighbours that are its own ghost (a cell
@@ -562,6 +581,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
             sb = limit_slope<R, LIMITER_MC>((fp - fb0) * inv_h, (fpp - fp) * inv_h);
           }
         } else {
+          const R inv_2h = R(grid_const<ONE>(ydir ? g.inv_2dy : g.inv_2dx));
           sa = (fp - fm) * inv_2h;
           sb = (fpp - fb0) * inv_2h;
         }
@@ -628,6 +648,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
       }
       mood_resets += reset ? 1u : 0u;
       // compute_fluxes, rotated for y faces (src/main.f90:394-401)
+      const R gamma = R(grid_const<ONE>(g.gamma));
+      const double rcp_gm1 = grid_const<ONE>(g.rcp_gm1);
       Flux5<R> F = riemann<R, SOLVER>(gamma, L[0], Rv[0], L[1], Rv[1], L[2], Rv[2], L[3], Rv[3], L[4], Rv[4], L[5],
                                       Rv[5], rcp_gm1);
       R* dst = (ydir ? sFy : sFx) + ff;
@@ -652,15 +674,9 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
     R* __restrict__ out[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      if constexpr (ONE) {
-        in[q] = static_cast<const R*>(g.buf[in_buf][q]);
-        u0[q] = static_cast<const R*>(g.buf[sbuf][q]);
-        out[q] = static_cast<R*>(g.buf[out_buf][q]);
-      } else {
-        in[q] = static_cast<const R*>(load_ptr(&g.buf[in_buf][q]));
-        u0[q] = static_cast<const R*>(load_ptr(&g.buf[sbuf][q]));
-        out[q] = static_cast<R*>(load_ptr(&g.buf[out_buf][q]));
-      }
+      in[q] = static_cast<const R*>(g.buf[in_buf][q]);
+      u0[q] = static_cast<const R*>(g.buf[sbuf][q]);
+      out[q] = static_cast<R*>(g.buf[out_buf][q]);
     }
 
     // ---- phase 3a: constrained transport -> new face B ------------------------
@@ -681,7 +697,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
       const R right = right_own ? fb : FBxY[yi + 1];
       return R(0.25) * (((-fa - up) + fb) + right);
     };
-    const R inv_dx = R(g.inv_dx), inv_dy = R(g.inv_dy);
+    const R inv_dx = R(grid_const<ONE>(g.inv_dx)), inv_dy = R(grid_const<ONE>(g.inv_dy));
+    const R dt = R(ctl->dt);
     const int bx_lo = (STAGE == 3 && (i0 > 0 || px)) ? -1 : 0;   // halo face column for the epilogue
     const int by_lo = (STAGE == 3 && (j0 > 0 || py)) ? -1 : 0;
     // (a taped stage 3 is run for what its floors change: it writes no state)
@@ -726,8 +743,9 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
     // ---- phase 3b: cell update -------------------------------------------------
     double e_speed = 0.0, e_dmax = 0.0, e_dsum = 0.0, e_bmax = 0.0, e_mass = 0.0, e_en = 0.0;
     unsigned floor_hits = 0;
-    const R ax = dt * R(g.dy);   // x-face weight (dt*dx in the square reference)
-    const R ay = dt * R(g.dx);
+    const R ax = dt * R(grid_const<ONE>(g.dy));   // x-face weight (dt*dx in the square reference)
+    const R ay = dt * R(grid_const<ONE>(g.dx));
+    const R gamma = R(grid_const<ONE>(g.gamma)), vol = R(grid_const<ONE>(g.vol));
     for (int c = tid; c < TX * TY; c += NT) {
       const int li = c % TX, lj = c / TX;
       const int i = i0 + li, j = j0 + lj;
@@ -827,10 +845,10 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
         const double Bx = hx ? 0.5 * (double(bxn) + double(bxm)) : double(bxn);
         const double By = hy ? 0.5 * (double(byn) + double(bym)) : double(byn);
         Prim<double> pr = get_primitive<double>(double(U[0]), double(U[1]), double(U[2]), double(U[3]),
-                                                Bx, By, g.gamma, g.vol, g.rcp_vol);
-        e_speed = run_max(e_speed, cfl_speed(pr.rho, pr.vx, pr.vy, pr.P, Bx, By, g.gamma));
+                                                Bx, By, gamma, vol, grid_const<ONE>(g.rcp_vol));
+        e_speed = run_max(e_speed, cfl_speed(pr.rho, pr.vx, pr.vy, pr.P, Bx, By, gamma));
         const double d = fabs(divb_cell(double(bxn), double(bxm), double(byn), double(bym), hx, hy,
-                                        g.inv_dx, g.inv_dy, g.square != 0));
+                                        inv_dx, inv_dy, g.square != 0));
         e_dmax = run_max(e_dmax, d);
         e_dsum += d;
         e_bmax = run_max(e_bmax, Bx * Bx + By * By);   // |B|^2 (root taken once, at the finish)
