@@ -542,10 +542,11 @@ static std::vector<int> small_variants(const chimera_handle* h) {
 // else variant 0 (Rusanov 994, 995 on 10; HLLE 1042, 1075), since they spill more at 80
 // registers.  FP32-bulk: variant 9, the 32 x 16 tile at three CTAs
 // an SM with TMA loads, the fastest for every solver (Kelvin-Helmholtz 4096^2
-// HLLD 4.84 ms a step against variant 0's 5.50, 2048^2 Rusanov 0.970 against
-// 1.134, rotor 1024^2 HLLE 280 us against 292).  FP32 on FP64 storage: variant
-// 1, three CTAs an SM (rotor 369 us against 382), but for HLLD, whose stage-2
-// and stage-3 fluxes that tile contracts differently in the last bit, variant 0.
+// HLLD 4.59 ms a step, 5.50 on variant 0, 5.09 without TMA; 2048^2 Rusanov 0.918,
+// 1.134, 1.030; rotor 1024^2 HLLE 252 us, 292, 284).  FP32 on FP64 storage: variant 1,
+// three CTAs an SM (rotor 318 us, 367 on variant 0; Kelvin-Helmholtz 2048^2 1.37 ms,
+// 1.58), but for HLLD batches, whose stage-2 and stage-3 fluxes that tile's general
+// kernel contracts differently in the last bit, variant 0.
 static int default_variant(const chimera_handle* h) {
   if (h->variants.size() == 1) return 0;
   for (int v : small_variants(h)) {
@@ -554,7 +555,7 @@ static int default_variant(const chimera_handle* h) {
     if (tiles <= std::min(resident_ctas(h, k[0]), std::min(resident_ctas(h, k[1]), resident_ctas(h, k[2])))) return v;
   }
   if (h->precision == CHIMERA_FP32_BULK) return 9;
-  if (h->precision == CHIMERA_FP32_MIXED) return h->riemann == CHIMERA_RIEMANN_HLLD ? 0 : 1;
+  if (h->precision == CHIMERA_FP32_MIXED) return (h->n > 1 && h->riemann == CHIMERA_RIEMANN_HLLD) ? 0 : 1;
   if (h->riemann == CHIMERA_RIEMANN_HLLD) return 11;
   if (h->n > 1) return 0;
   auto fullest = [&](int v) {   // cells of the SM that gets the most tiles

@@ -118,11 +118,11 @@ template <int TX, int TY> struct TmaBox64 {
 // Issued at the start of the current tile so the next tile's phase-1 loads
 // hit L2 instead of HBM.  Pure hints: no result, no synchronisation.  With
 // inputs = false only the U^n rows are prefetched (the inputs come by TMA).
-template <typename R, int TX, int TY, int NT, int STAGE>
+template <typename R, int TX, int TY, int NT, int STAGE, bool ONE>
 __device__ __forceinline__ void prefetch_next_tile(const StageArgs& a, int w_next, bool inputs = true) {
   if (w_next >= a.total_tiles) return;
-  const int m = (a.n_members == 1) ? 0 : a.tile_member[w_next];
-  const Member& g = a.members[m];
+  const int m = (ONE || a.n_members == 1) ? 0 : a.tile_member[w_next];
+  const Member& g = ONE ? a.one : a.members[m];
   const Control* ctl = a.ctl + m;
   const int nx = g.nx, ny = g.ny;
   const int lt = w_next - g.tile_begin;

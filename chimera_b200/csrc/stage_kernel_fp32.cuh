@@ -175,10 +175,10 @@ __device__ __forceinline__ Flux5<float> rusanov_x2(float gamma, float rho_L, flo
 
 // Whether work item w's input box lies inside its member's arrays (and the
 // member has tensor maps): then it is loaded by TMA.
-template <int TX, int TY, int BW, int BH>
+template <int TX, int TY, int BW, int BH, bool ONE>
 __device__ __forceinline__ bool tma_tile(const StageArgs& a, int w) {
-  const int m = (a.n_members == 1) ? 0 : a.tile_member[w];
-  const Member& g = a.members[m];
+  const int m = (ONE || a.n_members == 1) ? 0 : a.tile_member[w];
+  const Member& g = ONE ? a.one : a.members[m];
   if (!g.tmap) return false;
   const int lt = w - g.tile_begin;
   const int i0 = (lt % g.tiles_x) * TX, j0 = (lt / g.tiles_x) * TY;
@@ -186,10 +186,10 @@ __device__ __forceinline__ bool tma_tile(const StageArgs& a, int w) {
 }
 
 // Thread 0: issue the six box loads of work item w's stage input.
-template <int STAGE, int TX, int TY, int BW, int BH, int BOXF>
+template <int STAGE, int TX, int TY, int BW, int BH, int BOXF, bool ONE>
 __device__ __forceinline__ void tma_issue(const StageArgs& a, int w, float* stg, uint64_t* bar) {
-  const int m = (a.n_members == 1) ? 0 : a.tile_member[w];
-  const Member& g = a.members[m];
+  const int m = (ONE || a.n_members == 1) ? 0 : a.tile_member[w];
+  const Member& g = ONE ? a.one : a.members[m];
   const int lt = w - g.tile_begin;
   const int i0 = (lt % g.tiles_x) * TX, j0 = (lt / g.tiles_x) * TY;
   const int sbuf = a.ctl[m].parity;
@@ -200,9 +200,13 @@ __device__ __forceinline__ void tma_issue(const StageArgs& a, int w, float* stg,
   for (int q = 0; q < 6; ++q) tma_load_2d(stg + q * BOXF, maps + q * TMAP_BYTES, i0 - 4, j0 - 3, bar);
 }
 
+// ONE: a single grid, its descriptor in the launch, as in stage_kernel (at 80
+// registers 12 bytes of spills instead of 36; rotor 1024^2 272 -> 252 us a step,
+// Kelvin-Helmholtz 4096^2 4.89 -> 4.59 ms, on FP64 storage 361 -> 318 us and at 2048^2
+// 1.46 -> 1.37 ms).
 template <int SOLVER, int STAGE, int TX, int TY, int NT, int MINB, bool TMA, typename S = float,
-          bool MIXBC = false>
-__global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
+          bool MIXBC = false, bool ONE = false>
+__global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(const __grid_constant__ StageArgs a) {
   using G = TileGeom32<TX, TY>;
   static_assert(!TMA || G::TMA_FITS, "TMA staging must fit in the slope arrays");
   constexpr bool MIX = sizeof(S) == 8;   // FP64 storage, FP32 flux arithmetic
@@ -241,16 +245,16 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
     if (tid == 0) {
       mbar_init(&s_bar, 1);
       const int w0 = a.work_begin + int(blockIdx.x);
-      const bool st = w0 < a.total_tiles && tma_tile<TX, TY, G::BW, G::BH>(a, w0);
+      const bool st = w0 < a.total_tiles && tma_tile<TX, TY, G::BW, G::BH, ONE>(a, w0);
       s_tma = st ? 1u : 0u;
-      if (st) tma_issue<STAGE, TX, TY, G::BW, G::BH, G::BOXF>(a, w0, staging(), &s_bar);
+      if (st) tma_issue<STAGE, TX, TY, G::BW, G::BH, G::BOXF, ONE>(a, w0, staging(), &s_bar);
     }
     __syncthreads();
   }
 
   for (int w = a.work_begin + blockIdx.x; w < a.total_tiles; w += gridDim.x) {
-    const int m = (a.n_members == 1) ? 0 : a.tile_member[w];
-    const Member& g = a.members[m];
+    const int m = (ONE || a.n_members == 1) ? 0 : a.tile_member[w];
+    const Member& g = ONE ? a.one : a.members[m];
     Control* ctl = a.ctl + m;
     if (ctl->active == 0) {
       if (TMA && (s_tma & 1u)) {   // a copy was issued for this tile: consume it to keep the phases paired
@@ -304,8 +308,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
     }
     {
       const int wn = w + gridDim.x;   // the next tile's inputs are prefetched to L2 unless TMA loads them
-      prefetch_next_tile<S, TX, TY, NT, STAGE>(
-          a, wn, !(TMA && wn < a.total_tiles && tma_tile<TX, TY, G::BW, G::BH>(a, wn)));
+      prefetch_next_tile<S, TX, TY, NT, STAGE, ONE>(
+          a, wn, !(TMA && wn < a.total_tiles && tma_tile<TX, TY, G::BW, G::BH, ONE>(a, wn)));
     }
 
     // ---- phase 1: primitives (FP64 pressure recovery) -------------------------
@@ -563,11 +567,11 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
         const unsigned st = s_tma;     // this tile's state (every thread read it before phase 1's barrier)
         const unsigned parity = ((st >> 1) ^ st) & 1u;   // flips if this tile consumed a completion
         const int wn = w + gridDim.x;
-        const bool next = wn < a.total_tiles && tma_tile<TX, TY, G::BW, G::BH>(a, wn);
+        const bool next = wn < a.total_tiles && tma_tile<TX, TY, G::BW, G::BH, ONE>(a, wn);
         s_tma = (next ? 1u : 0u) | (parity << 1);
         if (next) {
           fence_proxy_async_smem();
-          tma_issue<STAGE, TX, TY, G::BW, G::BH, G::BOXF>(a, wn, staging(), &s_bar);
+          tma_issue<STAGE, TX, TY, G::BW, G::BH, G::BOXF, ONE>(a, wn, staging(), &s_bar);
         }
       }
     }
@@ -577,9 +581,9 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(StageArgs a) {
       // phases 1.5 and 2 (as the FP64 kernel does)
 #pragma unroll
       for (int q = 0; q < 6; ++q) {
-        in[q] = static_cast<const S*>(load_ptr(&g.buf[in_buf][q]));
-        u0[q] = static_cast<const S*>(load_ptr(&g.buf[sbuf][q]));
-        out[q] = static_cast<S*>(load_ptr(&g.buf[out_buf][q]));
+        in[q] = static_cast<const S*>(ONE ? g.buf[in_buf][q] : load_ptr(&g.buf[in_buf][q]));
+        u0[q] = static_cast<const S*>(ONE ? g.buf[sbuf][q] : load_ptr(&g.buf[sbuf][q]));
+        out[q] = static_cast<S*>(ONE ? g.buf[out_buf][q] : load_ptr(&g.buf[out_buf][q]));
       }
     }
 

@@ -10,7 +10,7 @@ from tests.gpu_util import require_gpu
 pytestmark = pytest.mark.gpu
 
 # the form's large-grid tile, by solver
-LARGE = {FP64: lambda r: 11 if r == HLLD else 10, FP32_BULK: lambda r: 9, FP32_MIXED: lambda r: 0 if r == HLLD else 1}
+LARGE = {FP64: lambda r: 11 if r == HLLD else 10, FP32_BULK: lambda r: 9, FP32_MIXED: lambda r: 1}
 
 
 @pytest.fixture(scope="module")
