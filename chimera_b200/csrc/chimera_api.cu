@@ -161,6 +161,7 @@ struct chimera_handle {
   char* d_tmaps = nullptr;           // [TMA variant slot][member][buffer 3][field 6] tensor maps
   std::vector<int> tmap_slot;        // per variant: its slot in d_tmaps, -1 without TMA
   std::vector<unsigned char> tmap_ok;   // [slot][member]: the member's maps exist
+  std::vector<unsigned char> tmap_built;   // [slot]: written
   // chimera_step_host: U^{n+1} goes back in chunks of tile rows on
   // copy_stream while the later chunks compute; stages 2 and 3 run on
   // band_stream[0] / [1] so that the chunks' partial waves of CTAs overlap.
@@ -310,6 +311,8 @@ static int launch_raw(chimera_handle* h, const KernelEntry& k, int grid, int w_b
 // CTAs of kernel k that the device holds at once.
 static int resident_ctas(const chimera_handle* h, const KernelEntry& k) {
   int per_sm = 0;
+  // every kernel that is launched comes through here (layout) first
+  cudaFuncSetAttribute(kernel_of(h, k), cudaFuncAttributeMaxDynamicSharedMemorySize, int(k.smem));
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel_of(h, k), k.nt, k.smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   cudaGetLastError();
@@ -479,10 +482,27 @@ static int layout(chimera_handle* h, int v) {
     tiles += g.tiles_x * g.tiles_y;
   }
   h->total_tiles = tiles;
-  // TMA variants: the variant's tensor maps (encoded once at creation and never
-  // modified) for the members whose shape allows them; the others, and every
-  // edge tile, use plain loads
+  // TMA variants: the variant's tensor maps (encoded the first time it is laid out
+  // and never modified) for the members whose shape allows them; the others, and
+  // every edge tile, use plain loads
   const int slot = h->tmap_slot.empty() ? -1 : h->tmap_slot[v];
+  if (slot >= 0 && !h->tmap_built[slot]) {
+    std::vector<unsigned char> maps(size_t(h->n) * 18 * TMAP_BYTES_HOST, 0);
+    const int bw = h->ks.stage[0][0].box_w, bh = h->ks.stage[0][0].box_h;
+    for (int m = 0; m < h->n; ++m) {
+      const Member& g = h->hm[m];
+      bool ok = true;
+      for (int b = 0; b < 3 && ok; ++b)
+        for (int q = 0; q < 6 && ok; ++q)
+          ok = encode_field_map(&maps[(size_t(m) * 18 + b * 6 + q) * TMAP_BYTES_HOST], g.buf[b][q], g.nx, g.ny, bw, bh,
+                                h->ks.elem_bytes);
+      h->tmap_ok[size_t(slot) * h->n + m] = ok ? 1 : 0;
+    }
+    CK(cudaMemcpyAsync(h->d_tmaps + size_t(slot) * maps.size(), maps.data(), maps.size(), cudaMemcpyHostToDevice,
+                       h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    h->tmap_built[slot] = 1;
+  }
   for (int m = 0; m < h->n; ++m)
     h->hm[m].tmap = (slot >= 0 && h->tmap_ok[size_t(slot) * h->n + m])
                         ? h->d_tmaps + (size_t(slot) * h->n + m) * 18 * TMAP_BYTES_HOST
@@ -627,12 +647,7 @@ int chimera_batch_create(int n_members, const chimera_cfg* cfgs, void* stream, c
     else if (h->precision == CHIMERA_FP64) fp64_kernels(v, &h->variants[v]);
     else if (h->precision == CHIMERA_FP32_BULK) fp32_kernels(v, &h->variants[v]);
     else fp32m_kernels(v, &h->variants[v]);
-    for (int r = 0; r < 3; ++r)
-      for (int st = 0; st < 3; ++st)
-        cudaFuncSetAttribute(kernel_of(h, h->variants[v].stage[r][st]), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(h->variants[v].stage[r][st].smem));
   }
-  cudaGetLastError();
   h->ks = h->variants[0];
   if (stream) {
     h->stream = (cudaStream_t)stream;
@@ -702,32 +717,15 @@ int chimera_batch_create(int n_members, const chimera_cfg* cfgs, void* stream, c
     chimera_destroy(h);
     return CHIMERA_ERR_NOMEM;
   }
-  // tensor maps of every TMA variant, written once here and never modified
+  // room for every TMA variant's tensor maps (written by the first layout that uses them)
   h->tmap_slot.assign(nv, -1);
   int slots = 0;
   for (int v = 0; v < nv; ++v)
     if (h->variants[v].stage[0][0].box_w > 0) h->tmap_slot[v] = slots++;
   if (slots > 0) {
-    const size_t per_slot = size_t(n_members) * 18 * TMAP_BYTES_HOST;
-    std::vector<unsigned char> maps(per_slot * slots, 0);
     h->tmap_ok.assign(size_t(slots) * n_members, 0);
-    for (int v = 0; v < nv; ++v) {
-      const int sl = h->tmap_slot[v];
-      if (sl < 0) continue;
-      const int bw = h->variants[v].stage[0][0].box_w, bh = h->variants[v].stage[0][0].box_h;
-      for (int m = 0; m < n_members; ++m) {
-        const Member& g = h->hm[m];
-        bool ok = true;
-        for (int b = 0; b < 3 && ok; ++b)
-          for (int q = 0; q < 6 && ok; ++q)
-            ok = encode_field_map(&maps[sl * per_slot + (size_t(m) * 18 + b * 6 + q) * TMAP_BYTES_HOST],
-                                  g.buf[b][q], g.nx, g.ny, bw, bh, h->variants[v].elem_bytes);
-        h->tmap_ok[size_t(sl) * n_members + m] = ok ? 1 : 0;
-      }
-    }
-    if (cudaMalloc(&h->d_tmaps, maps.size()) != cudaSuccess ||
-        cudaMemcpyAsync(h->d_tmaps, maps.data(), maps.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
-        cudaStreamSynchronize(h->stream) != cudaSuccess) {
+    h->tmap_built.assign(slots, 0);
+    if (cudaMalloc(&h->d_tmaps, size_t(slots) * n_members * 18 * TMAP_BYTES_HOST) != cudaSuccess) {
       cudaGetLastError();
       chimera_destroy(h);
       return CHIMERA_ERR_NOMEM;
