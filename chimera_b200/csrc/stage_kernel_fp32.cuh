@@ -473,7 +473,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(const __grid_consta
         unsigned outside = 0;   // bit q: a state of field q is not between the low and the high cell's values
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
-          const R f0 = sP[q * G::NP + pa], fp = sP[q * G::NP + pb];
+          const R f0 = sP[q * G::NP + pa];
+          R fp = sP[q * G::NP + pb];
           // left and right states as the two lanes of one paired FP32 multiply-add
           const float2 v = __ffma2_rn(make_float2(hh, -hh),
                                       make_float2(sS[(2 * q + d) * G::NS + c], sS[(2 * q + d) * G::NS + sb]),
@@ -483,9 +484,10 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_f32(const __grid_consta
           if constexpr (MIXBC) {
             // the face below x = 0 (y = 0) with that side periodic and the far
             // side outflow is the far side's outflow face: its high cell is the
-            // low cell's own ghost (value f0, zero slope)
+            // low cell's own ghost (value f0, zero slope), which is also the high
+            // cell of the bounds
             const int gl = ydir ? j0 + cy - 1 : i0 + cx - 1;
-            if (gl == -1 && (ydir ? (py && !pyh) : (px && !pxh))) vR = f0;
+            if (gl == -1 && (ydir ? (py && !pyh) : (px && !pxh))) vR = fp = f0;
           }
           // The low and the high cell are two of the five cells of the MOOD bounds
           // below: states between their two values (with the rho / P floor on the
