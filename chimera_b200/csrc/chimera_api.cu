@@ -16,6 +16,7 @@
 #include <mutex>
 #include <new>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -470,6 +471,7 @@ static int tiles_for(const chimera_handle* h, int tx, int ty) {
 // Switch the tile decomposition to variant v: member tiling, work list and
 // persistent grid sizes (descriptors are re-uploaded; state is untouched).
 static int layout(chimera_handle* h, int v) {
+  if (v < 0 || v >= int(h->variants.size())) return CHIMERA_ERR_BAD_ARG;
   h->ks = h->variants[v];
   h->cur_variant = v;
   const int tx = h->ks.stage[0][0].tx, ty = h->ks.stage[0][0].ty;
@@ -519,8 +521,9 @@ static int layout(chimera_handle* h, int v) {
   return CHIMERA_OK;
 }
 
-// Autotuner results per problem shape, shared by the handles of a process.
-using TuneKey = std::tuple<int, int, int, int, int, long long, int>;
+// Autotuner results per problem shape, shared by the handles of a process: the
+// switches, the number of variants (a mixed pair has one) and the members' sizes.
+using TuneKey = std::tuple<int, int, int, int, int, int, std::vector<std::pair<int, int>>>;
 static std::map<TuneKey, int>& tune_cache() {
   static std::map<TuneKey, int> c;
   return c;
@@ -530,9 +533,10 @@ static std::mutex& tune_mutex() {
   return m;
 }
 static TuneKey tune_key(const chimera_handle* h) {
-  long long cells = 0;
-  for (int m = 0; m < h->n; ++m) cells += (long long)cells_of(h->cfg[m]);
-  return TuneKey(h->precision, h->riemann, h->limiter, h->mood, h->slope, cells, h->n);
+  std::vector<std::pair<int, int>> sizes;
+  for (const chimera_cfg& c : h->cfg) sizes.emplace_back(c.nx, c.ny);
+  std::sort(sizes.begin(), sizes.end());   // (the members' order does not matter)
+  return TuneKey(h->precision, h->riemann, h->limiter, h->mood, h->slope, int(h->variants.size()), std::move(sizes));
 }
 
 // The small-grid variants of a precision, smallest tile first.

@@ -1,0 +1,58 @@
+"""The library's host side without a GPU: the CUDA runtime replaced by
+fake_cudart.c, in a child process."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+@pytest.fixture(scope="module")
+def child(tmp_path_factory):
+    from chimera_b200 import build, gpu
+    if not os.path.exists(gpu.LIB_PATH):
+        build.build()
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    include = os.path.join(os.path.dirname(os.path.dirname(build._nvcc())), "include")
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", "-I" + include, "-o", so, os.path.join(HERE, "fake_cudart.c")],
+                   check=True)
+    head = f"""
+import ctypes as C, sys
+sys.path.insert(0, {ROOT!r})
+from chimera_b200 import gpu
+from chimera_b200.config import *
+fake = C.CDLL(None)
+fake.fake_live_bytes.restype = C.c_longlong
+lib = gpu.lib()
+def grid(nx, ny=None, **kw):
+    return SolverConfig(nx=nx, ny=ny or nx, dx=1.0 / nx, dy=1.0 / nx, gamma=5.0 / 3.0, **kw)
+"""
+
+    def run(body):
+        r = subprocess.run([sys.executable, "-c", head + body], env=dict(os.environ, LD_PRELOAD=so), capture_output=True,
+                           text=True, timeout=120)
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+def test_autotuned_choice_stays_with_its_shape(child):
+    """A tile chosen for one problem is not taken for another one of as many cells: a
+    mixed pair of sides, which has one tile, or another shape."""
+    child("""
+ms = (C.c_float * 64)(*([5.0] * 3 + [1.0] + [5.0] * 60))
+fake.fake_elapsed(ms, 64)
+with gpu.Solver(grid(64, bc=(BC_PERIODIC,) * 4)) as s:
+    default = s.variant()["variant"]
+    chosen, _ = s.autotune(1)
+    assert chosen == 3 != default
+with gpu.Solver(grid(64, bc=(BC_OUTFLOW,) * 4)) as s:
+    assert s.variant()["variant"] == 3
+with gpu.Solver(grid(64, bc=(BC_PERIODIC, BC_OUTFLOW, BC_PERIODIC, BC_PERIODIC))) as s:
+    assert s.variant_count() == 1 and s.variant()["variant"] == 0
+    s.step(1)
+with gpu.Solver(grid(32, 128)) as s:
+    assert s.variant()["variant"] == default
+""")
