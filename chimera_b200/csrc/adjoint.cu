@@ -419,6 +419,17 @@ __device__ __forceinline__ void slope_vjp(const AdjGeom& g, double dl, double dr
   }
 }
 
+// Where the magnetic floor X cut a recovered pressure, or ties with it: derivatives of
+// the pressure w.r.t. the recovered value (from the quotient E / vol, rounded
+// once as the forward rounds it) and w.r.t. X.  Rare: kept out of line.
+__device__ __noinline__ double2 cut_pressure_weights(double E, double vol, double ke, double hB, double gm1,
+                                                    double X) {
+  const double P0 = ((E / vol - ke) - hB) * gm1 + hB;
+  const bool warm = P0 > K<double>::P_floor;
+  const double w = max_weight(warm ? P0 : K<double>::P_floor, X);
+  return make_double2(warm ? w : 0.0, 1.0 - w);
+}
+
 __device__ __forceinline__ int wrap_far(int p, int n) {   // any p >= -n
   while (p < 0) p += n;
   while (p >= n) p -= n;
@@ -571,18 +582,18 @@ __global__ void __launch_bounds__(RC_NT, 2) k_rev_cells(const __grid_constant__ 
       const double r = a.tape.P[0][c], u = a.tape.P[1][c], v = a.tape.P[2][c];
       const double Bx = a.tape.P[4][c], By = a.tape.P[5][c];
       const double gm1 = g.gamma - 1.0, hB = 0.5 * (Bx * Bx + By * By), vv = u * u + v * v, ke = 0.5 * r * vv;
-      const double P0 = ((a.U[3][c] * g.ivol - ke) - hB) * gm1 + hB;
-      const bool warm = P0 > K<double>::P_floor;
-      const double P1 = warm ? P0 : K<double>::P_floor;
-      const double X = hB + K<double>::e_floor_frac * (ke + hB);
-      const double wP = max_weight(P1, X);
-      const double aX = (1.0 - wP) * lP[3], a0 = warm ? wP * lP[3] : 0.0;
+      // The branches the recovery took, from what it left: its pressure is above X where
+      // it was not cut by it, its density above the floor where the mass was.
+      const double P = a.tape.P[3][c], X = hB + K<double>::e_floor_frac * (ke + hB);
+      double2 w = make_double2(P > K<double>::P_floor ? 1.0 : 0.0, 0.0);
+      if (!(P > X)) w = cut_pressure_weights(a.U[3][c], g.vol, ke, hB, gm1, X);
+      const double a0 = w.x * lP[3], aX = w.y * lP[3];
       const double ake = K<double>::e_floor_frac * aX - a0 * gm1;
       const double ahB = (1.0 + K<double>::e_floor_frac) * aX + a0 * (1.0 - gm1);
       const double ir = 1.0 / r, im = ir * g.ivol;
       const double au = lP[1] + ake * r * u, av = lP[2] + ake * r * v;
       const double ar = lP[0] + ake * (0.5 * vv) - (au * u + av * v) * ir;
-      lin[0] = (a.U[0][c] * g.ivol > K<double>::rho_floor) ? ar * g.ivol : 0.0;
+      lin[0] = (r > K<double>::rho_floor) ? ar * g.ivol : 0.0;
       lin[1] = au * im;
       lin[2] = av * im;
       lin[3] = a0 * gm1 * g.ivol;
