@@ -97,6 +97,21 @@ struct NvtxRange {
 };
 const char* const kLaunchName[4] = {"chimera cfl", "chimera stage 1", "chimera stage 2", "chimera stage 3"};
 
+// The handle's device for the span of a call whose kernels the caller may not have
+// selected it for: a launch on a stream of another device than the current one fails.
+struct DeviceGuard {
+  int old = -1;
+  explicit DeviceGuard(int dev) {
+    int cur = dev;
+    if (cudaGetDevice(&cur) == cudaSuccess && cur != dev && cudaSetDevice(dev) == cudaSuccess) old = cur;
+  }
+  ~DeviceGuard() {
+    if (old >= 0) cudaSetDevice(old);
+  }
+  DeviceGuard(const DeviceGuard&) = delete;
+  DeviceGuard& operator=(const DeviceGuard&) = delete;
+};
+
 // cuTensorMapEncodeTiled from the driver, through the runtime (the library
 // links only cudart); null if the driver does not provide it.
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -844,6 +859,7 @@ int chimera_batch_set_state(chimera_handle* h, int m, const double* Mass, const 
   const void* ptrs[6] = {Mass, Momx, Momy, Energy, b_x, b_y};
   int rc = check_io(h, m, ptrs, ld, where);
   if (rc) return rc;
+  DeviceGuard on(h->device);
   if (movable(h, ptrs, where)) {
     // one kernel, once the work before it is done: the arrays are read right away
     CK(cudaStreamSynchronize(h->stream));
@@ -874,6 +890,7 @@ static int get_buffer(chimera_handle* h, int m, int which, double* const* ptrs, 
   const void* p6[6] = {ptrs[0], ptrs[1], ptrs[2], ptrs[3], ptrs[4], ptrs[5]};
   int rc = check_io(h, m, p6, ld, where);
   if (rc) return rc;
+  DeviceGuard on(h->device);
   Control c;
   if (movable(h, p6, where)) {   // one kernel and one wait
     rc = move_state<false>(h, m, which, p6, ld);
@@ -1048,6 +1065,7 @@ int chimera_step_host(chimera_handle* h, const double* const* in, double* const*
 
 int chimera_batch_set_time(chimera_handle* h, int m, double t, int output_count) {
   if (!h || m < 0 || m >= h->n || output_count < 1) return CHIMERA_ERR_BAD_ARG;
+  DeviceGuard on(h->device);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CK(cudaStreamIsCapturing(h->stream, &cs));
   if (cs != cudaStreamCaptureStatusNone) return CHIMERA_ERR_CUDA;   // dt_valid is the host's: not for a replay

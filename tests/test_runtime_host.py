@@ -56,3 +56,23 @@ with gpu.Solver(grid(64, bc=(BC_PERIODIC, BC_OUTFLOW, BC_PERIODIC, BC_PERIODIC))
 with gpu.Solver(grid(32, 128)) as s:
     assert s.variant()["variant"] == default
 """)
+
+
+@pytest.mark.parametrize("precision", ["FP64", "FP32_BULK", "FP32_MIXED"])
+def test_state_and_time_with_another_device_current(child, precision):
+    """set_state, get_state and set_time of a handle whose device is not the current one:
+    done on the handle's device, the caller's choice left as it was."""
+    child(f"""
+with gpu.Solver(grid(16, precision={precision})) as s:
+    dev = [C.c_void_p() for _ in range(6)]
+    for d in dev:
+        assert fake.cudaMalloc(C.byref(d), C.c_size_t(16 * 16 * 8)) == 0
+    assert fake.cudaSetDevice(1) == 0
+    assert lib.chimera_batch_set_state(s.handle, 0, *dev, 16, gpu.DEVICE) == 0
+    assert lib.chimera_batch_get_state(s.handle, 0, *dev, 16, gpu.DEVICE) == 0
+    assert fake.fake_launches(b"move_state_kernel") == 2
+    assert lib.chimera_batch_set_time(s.handle, 0, 0.5, 2) == 0
+    assert fake.fake_launches(b"set_time_kernel") == 1
+    now = C.c_int()
+    assert fake.cudaGetDevice(C.byref(now)) == 0 and now.value == 1
+""")
