@@ -176,6 +176,11 @@ class Solver:
         _check(lib().chimera_batch_create(len(self.cfgs), arr, C.c_void_p(stream), C.byref(h)),
                "chimera_batch_create")
         self._h = h
+        self._raw = self.stream
+        dev = C.c_int()
+        lib().cudaGetDevice(C.byref(dev))   # (the runtime the library is linked with)
+        self._device = dev.value
+        self._ext = None                    # the solver's stream as a torch stream
 
     def close(self):
         if getattr(self, "_h", None):
@@ -203,32 +208,47 @@ class Solver:
     def stream(self) -> int:
         return lib().chimera_stream(self._h) or 0
 
-    def _after_torch(self, arrays):
-        """Order the solver's stream after torch's current one, where CUDA tensors
-        may still be written or read."""
+    def _torch_streams(self, arrays):
+        """(torch's current stream, the solver's) for every device of the arrays where they
+        are CUDA tensors and the two differ; nothing under a capture."""
         if not getattr(arrays[0], "is_cuda", False):
-            return
+            return []
         import torch
-        cur = torch.cuda.current_stream()
-        if cur.cuda_stream != self.stream and not torch.cuda.is_current_stream_capturing():
-            torch.cuda.ExternalStream(self.stream).wait_stream(cur)
+        out = []
+        for dev in {a.get_device() for a in arrays}:
+            if torch._C._cuda_getCurrentRawStream(dev) != self._raw and not torch.cuda.is_current_stream_capturing():
+                if self._ext is None:
+                    self._ext = torch.cuda.ExternalStream(self._raw, device=self._device)
+                out.append((torch.cuda.current_stream(dev), self._ext))
+        return out
+
+    @staticmethod
+    def _order(pairs):
+        """What is queued on the second stream of each pair comes before what follows on
+        the first."""
+        for first, second in pairs:
+            first.wait_stream(second)
 
     def set_state(self, arrays: Sequence, member: int = 0):
         """Six conserved fields (Mass, Momx, Momy, Energy, b_x, b_y) of member
         ``member`` in: numpy arrays or CPU tensors are read completely before
         the call returns (page-locked ones included); CUDA tensors are copied
-        in order on the solver's stream, after torch's current stream."""
+        in order on the solver's stream, after what is queued on torch's current
+        stream and before what is queued there next."""
         c = self.cfgs[member]
         p, ld, where, keep = _ptrs(arrays, c.nx, c.ny)
-        self._after_torch(arrays)
-        _check(lib().chimera_batch_set_state(self._h, member, *p, ld, where), "set_state")
+        streams = self._torch_streams(arrays)
+        self._order((ext, cur) for cur, ext in streams)
+        rc = lib().chimera_batch_set_state(self._h, member, *p, ld, where)
+        self._order(streams)
+        _check(rc, "set_state")
 
     def get_state(self, member: int = 0, out=None, check: bool = True):
         c = self.cfgs[member]
         if out is None:
             out = [np.empty((c.ny, c.nx), dtype=np.float64) for _ in range(6)]
         p, ld, where, keep = _ptrs(out, c.nx, c.ny, out=True)
-        self._after_torch(out)
+        self._order((ext, cur) for cur, ext in self._torch_streams(out))   # (the call waits for the copies)
         rc = lib().chimera_batch_get_state(self._h, member, *p, ld, where)
         if check:
             _check(rc, "get_state")

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from chimera_b200 import problems as P
+from chimera_b200.config import FP32_BULK, FP64
 from tests.gpu_util import require_gpu
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +54,35 @@ def test_adjoint_waits_for_the_tensors(A, side_stream):
             del gone, g
             adj.forward_step(U, 1e-4)
             assert all(torch.equal(a, b) for a, b in zip(kept, U))
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_BULK])
+@pytest.mark.parametrize("behind", [0, 5])
+def test_set_state_reads_before_later_writes(A, precision, behind):
+    """In-place writes queued after set_state, and new owners of a freed tensor's memory,
+    come after its read: of a state that takes longer to copy than the writes to start,
+    and of one whose copy waits for the solver's steps."""
+    from chimera_b200 import gpu
+    n = 4096
+    cfg, _ = P.orszag_tang(8)
+    cfg = cfg.replace(nx=n, ny=n, precision=precision)
+    U = [1.0 + torch.rand((n, n), dtype=torch.float64, device="cuda").float().double() for _ in range(6)]
+    got, want = ([torch.empty_like(u) for u in U] for _ in range(2))
+    with gpu.Solver(cfg) as s:
+        s.set_state(U)
+        torch.cuda.synchronize()
+        s.get_state(out=want)               # in the storage's precision
+        for freed in (False, True):
+            V = [u.clone() for u in U]
+            s.set_state(U)
+            s.set_time(0.0)
+            s.step(behind)
+            s.set_state(V)
+            if freed:
+                del V
+                V = [torch.empty_like(u) for u in U]
+            for v in reversed(V):
+                v.fill_(7.0)
+            s.get_state(out=got, check=False)
+            assert all(torch.equal(a, b) for a, b in zip(got, want)), freed
+            del V
