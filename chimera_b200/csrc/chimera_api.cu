@@ -442,7 +442,7 @@ static int run_steps(chimera_handle* h, int nsteps) {
 static size_t cells_of(const chimera_cfg& c) { return size_t(c.nx) * size_t(c.ny); }
 
 // Whether the six arrays can be moved by a kernel: float64-aligned memory of the
-// handle's device, and no capture under way (the calls wait for the device, which a
+// handle's device, and no capture under way (the copies wait for the device, which a
 // capture refuses, as it always has).
 static bool movable(chimera_handle* h, const void* const* ptrs, int where) {
   if (where != CHIMERA_DEVICE) return false;
@@ -860,9 +860,7 @@ int chimera_batch_set_state(chimera_handle* h, int m, const double* Mass, const 
   int rc = check_io(h, m, ptrs, ld, where);
   if (rc) return rc;
   DeviceGuard on(h->device);
-  if (movable(h, ptrs, where)) {
-    // one kernel, once the work before it is done: the arrays are read right away
-    CK(cudaStreamSynchronize(h->stream));
+  if (movable(h, ptrs, where)) {   // one kernel in the stream's order, without a wait
     h->dt_valid[m] = false;
     return move_state<true>(h, m, 0, ptrs, ld);
   }

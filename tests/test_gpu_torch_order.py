@@ -1,5 +1,6 @@
 """CUDA tensors that torch's stream is still writing, or writes next: every call takes
 them in torch's order."""
+import numpy as np
 import pytest
 import torch
 
@@ -86,3 +87,19 @@ def test_set_state_reads_before_later_writes(A, precision, behind):
             s.get_state(out=got, check=False)
             assert all(torch.equal(a, b) for a, b in zip(got, want)), freed
             del V
+
+
+def test_set_state_does_not_hold_the_host(A):
+    """Work queued on torch's stream delays the copy, not the caller."""
+    from chimera_b200 import gpu
+    cfg, st = P.orszag_tang(64)
+    U = [torch.from_numpy(x).cuda() for x in st]
+    with gpu.Solver(cfg) as s:
+        s.set_state(U)
+        torch.cuda.synchronize()
+        done = torch.cuda.Event()
+        V = _late(U)
+        done.record()
+        s.set_state(V)
+        assert not done.query()
+        assert all(np.array_equal(a, b) for a, b in zip(s.get_state(), st))
