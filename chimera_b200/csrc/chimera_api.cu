@@ -164,7 +164,8 @@ struct chimera_handle {
   KernelSet ks{};                    // the active variant's kernels
   std::vector<KernelSet> variants;
   int cur_variant = 0;
-  int max_tiles = 0;                 // over all variants (partials / work-list capacity)
+  int max_tiles = 0;                 // capacity of the partials and the work list (reserve_tiles)
+  std::vector<void*> outgrown;       // the smaller ones before them
   int dry = 0;
   int grid_stage[3] = {0, 0, 0};
   int grid_cfl = 0;
@@ -483,10 +484,31 @@ static int tiles_for(const chimera_handle* h, int tx, int ty) {
   return t;
 }
 
+// Room for the partials and the work list of `tiles` tiles.  What they replace is
+// kept until the handle goes, as everything else that a launch may hold.
+static int reserve_tiles(chimera_handle* h, int tiles) {
+  if (tiles <= h->max_tiles) return CHIMERA_OK;
+  void *part = nullptr, *member = nullptr;
+  if (cudaMalloc(&part, sizeof(double) * NPART * size_t(tiles)) != cudaSuccess ||
+      cudaMalloc(&member, sizeof(int) * size_t(tiles)) != cudaSuccess) {
+    cudaFree(part);
+    cudaGetLastError();
+    return CHIMERA_ERR_NOMEM;
+  }
+  if (h->d_part) h->outgrown.insert(h->outgrown.end(), {h->d_part, h->d_tile_member});
+  h->d_part = static_cast<double*>(part);
+  h->d_tile_member = static_cast<int*>(member);
+  h->max_tiles = tiles;
+  return CHIMERA_OK;
+}
+
 // Switch the tile decomposition to variant v: member tiling, work list and
 // persistent grid sizes (descriptors are re-uploaded; state is untouched).
 static int layout(chimera_handle* h, int v) {
   if (v < 0 || v >= int(h->variants.size())) return CHIMERA_ERR_BAD_ARG;
+  const KernelEntry& k0 = h->variants[v].stage[0][0];
+  const int rc = reserve_tiles(h, tiles_for(h, k0.tx, k0.ty));
+  if (rc) return rc;   // still on the variant before
   h->ks = h->variants[v];
   h->cur_variant = v;
   const int tx = h->ks.stage[0][0].tx, ty = h->ks.stage[0][0].ty;
@@ -681,10 +703,6 @@ int chimera_batch_create(int n_members, const chimera_cfg* cfgs, void* stream, c
   const int eb = h->ks.elem_bytes;
   h->hm.resize(n_members);
   size_t pool_bytes = 0;
-  int tiles = 0;
-  for (int v = 0; v < nv; ++v)
-    tiles = std::max(tiles, tiles_for(h, h->variants[v].stage[0][0].tx, h->variants[v].stage[0][0].ty));
-  h->max_tiles = tiles;
   for (int m = 0; m < n_members; ++m) {
     const chimera_cfg& c = cfgs[m];
     Member& g = h->hm[m];
@@ -712,6 +730,20 @@ int chimera_batch_create(int n_members, const chimera_cfg* cfgs, void* stream, c
     h->max_cells = std::max(h->max_cells, n);
     pool_bytes += 18 * ((n * eb + 255) / 256) * 256;
   }
+  int v0 = default_variant(h);
+  {
+    std::lock_guard<std::mutex> lk(tune_mutex());
+    auto it = tune_cache().find(tune_key(h));
+    if (it != tune_cache().end()) v0 = it->second;
+  }
+  // partials and work list for the tile the handle starts on and for every tile of 256
+  // cells or more (0.2 bytes a cell); the 8 x 8 and 16 x 8 tiles, which only small grids
+  // gain from, get theirs (0.8) when they are laid out
+  int tiles = 0;
+  for (int v = 0; v < nv; ++v) {
+    const KernelEntry& k = h->variants[v].stage[0][0];
+    if (v == v0 || k.tx * k.ty >= 256) tiles = std::max(tiles, tiles_for(h, k.tx, k.ty));
+  }
   h->dt_valid.assign(n_members, false);
   if (cudaMalloc(&h->pool, pool_bytes) != cudaSuccess) { cudaGetLastError(); chimera_destroy(h); return CHIMERA_ERR_NOMEM; }
   cudaMemsetAsync(h->pool, 0, pool_bytes, h->stream);
@@ -729,9 +761,7 @@ int chimera_batch_create(int n_members, const chimera_cfg* cfgs, void* stream, c
     ctl[m].active = 1;
   }
   if (cudaMalloc(&h->d_members, sizeof(Member) * n_members) != cudaSuccess ||
-      cudaMalloc(&h->d_ctl, sizeof(Control) * n_members) != cudaSuccess ||
-      cudaMalloc(&h->d_part, sizeof(double) * NPART * size_t(h->max_tiles)) != cudaSuccess ||
-      cudaMalloc(&h->d_tile_member, sizeof(int) * size_t(h->max_tiles)) != cudaSuccess) {
+      cudaMalloc(&h->d_ctl, sizeof(Control) * n_members) != cudaSuccess || reserve_tiles(h, tiles) != CHIMERA_OK) {
     cudaGetLastError();
     chimera_destroy(h);
     return CHIMERA_ERR_NOMEM;
@@ -759,12 +789,6 @@ int chimera_batch_create(int n_members, const chimera_cfg* cfgs, void* stream, c
   }
   cudaMemcpyAsync(h->d_ctl, ctl.data(), sizeof(Control) * n_members, cudaMemcpyHostToDevice, h->stream);
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) { cudaGetLastError(); chimera_destroy(h); return CHIMERA_ERR_CUDA; }
-  int v0 = default_variant(h);
-  {
-    std::lock_guard<std::mutex> lk(tune_mutex());
-    auto it = tune_cache().find(tune_key(h));
-    if (it != tune_cache().end()) v0 = it->second;
-  }
   if (layout(h, v0) != CHIMERA_OK) { chimera_destroy(h); return CHIMERA_ERR_CUDA; }
   *out = h;
   return CHIMERA_OK;
@@ -786,6 +810,7 @@ void chimera_destroy(chimera_handle* h) {
   cudaFree(h->d_ctl);
   cudaFree(h->d_part);
   cudaFree(h->d_tile_member);
+  for (void* p : h->outgrown) cudaFree(p);
   cudaFree(h->d_stage64);
   cudaFree(h->d_tmaps);
   for (auto e : h->band_done)
@@ -1250,6 +1275,10 @@ int chimera_autotune(chimera_handle* h, int reps, int* chosen, double* best_ms) 
         tiles_for(h, k.tx, k.ty) > 2 * resident_ctas(h, k))
       continue;
     rc = layout(h, v);
+    if (rc == CHIMERA_ERR_NOMEM) {   // no room for its work list: not a candidate
+      rc = CHIMERA_OK;
+      continue;
+    }
     if (rc) break;
     h->dry = 1;
     rc = one_step(h);                       // warm-up

@@ -14,6 +14,7 @@ static struct { const void* fn; const char* name; int launches; } kernels[MAX_KE
 static int n_kernels = 0;
 static struct { char* p; size_t n; int dev; } blocks[MAX_BLOCKS];
 static long long live = 0;                 /* bytes allocated and not freed */
+static long long limit = 1LL << 60;        /* bytes there are */
 static const float* elapsed = 0;           /* what the next event pairs measure */
 static int n_elapsed = 0;
 struct CUstream_st { int dev; };
@@ -21,6 +22,7 @@ struct CUevent_st { int dev; };
 
 /* what a test reads and sets */
 long long fake_live_bytes(void) { return live; }
+void fake_memory(long long bytes) { limit = bytes; }
 int fake_launches(const char* part) {      /* launches of kernels whose name holds part */
   int s = 0;
   for (int k = 0; k < n_kernels; ++k)
@@ -90,6 +92,7 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char* n, void** f, unsigned v
 
 /* memory */
 cudaError_t cudaMalloc(void** p, size_t n) {
+  if (live + (long long)n > limit) return cudaErrorMemoryAllocation;
   for (int k = 0; k < MAX_BLOCKS; ++k)
     if (!blocks[k].p) {
       if (!(*p = calloc(n ? n : 1, 1))) return cudaErrorMemoryAllocation;

@@ -76,3 +76,27 @@ with gpu.Solver(grid(16, precision={precision})) as s:
     now = C.c_int()
     assert fake.cudaGetDevice(C.byref(now)) == 0 and now.value == 1
 """)
+
+
+def test_work_list_memory_follows_the_tiles(child):
+    """A large grid holds partials and a work list for large tiles (52 bytes a tile of 256
+    cells: 0.21 a cell); a small tile gets its own when it is chosen, or the choice is
+    refused and the handle stays as it was."""
+    child("""
+cells = 1024 * 1024
+with gpu.Solver(grid(1024, precision=FP32_BULK)) as s:
+    state = 18 * 4 * cells + 8 * cells          # three buffer sets, the float64 staging
+    other = fake.fake_live_bytes() - state
+    assert 0 < other <= 0.21 * cells, other / cells
+    before = s.variant()
+    fake.fake_memory(C.c_longlong(fake.fake_live_bytes() + cells // 2))
+    assert lib.chimera_set_variant(s.handle, 11) == -7      # 8 x 8 tiles: 0.8 bytes a cell
+    assert s.variant() == before
+    s.step(1)
+    s.autotune(1)
+    fake.fake_memory(C.c_longlong(1 << 60))
+    s.set_variant(11)
+    assert s.variant()["tile"] == (8, 8) and fake.fake_live_bytes() - state >= 52 * cells // 64
+    s.step(1)
+assert fake.fake_live_bytes() == 0
+""")
