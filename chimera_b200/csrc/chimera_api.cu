@@ -1274,6 +1274,10 @@ int chimera_autotune(chimera_handle* h, int reps, int* chosen, double* best_ms) 
     if (std::find(small.begin(), small.end(), v) != small.end() &&
         tiles_for(h, k.tx, k.ty) > 2 * resident_ctas(h, k))
       continue;
+    // nor the kernels of an earlier variant (FP32 8 is 2 since the slopes' bounds went)
+    bool seen = false;
+    for (int e = 0; e < v; ++e) seen = seen || h->variants[e].stage[h->riemann - 1][0].fn == k.fn;
+    if (seen) continue;
     rc = layout(h, v);
     if (rc == CHIMERA_ERR_NOMEM) {   // no room for its work list: not a candidate
       rc = CHIMERA_OK;

@@ -29,9 +29,10 @@ int fake_launches(const char* part) {      /* launches of kernels whose name hol
     if (strstr(kernels[k].name, part)) s += kernels[k].launches;
   return s;
 }
-int fake_kernels_launched(void) {          /* how many different kernels ran */
+int fake_most_launches(void) {             /* of any one stage kernel */
   int s = 0;
-  for (int k = 0; k < n_kernels; ++k) s += kernels[k].launches > 0;
+  for (int k = 0; k < n_kernels; ++k)
+    if (strstr(kernels[k].name, "stage_kernel") && kernels[k].launches > s) s = kernels[k].launches;
   return s;
 }
 void fake_reset(void) { for (int k = 0; k < n_kernels; ++k) kernels[k].launches = 0; }

@@ -100,3 +100,15 @@ with gpu.Solver(grid(1024, precision=FP32_BULK)) as s:
     s.step(1)
 assert fake.fake_live_bytes() == 0
 """)
+
+
+def test_autotuner_times_a_kernel_once(child):
+    """Two variants that name the same kernels are one candidate: each stage kernel runs in
+    the warm-up step and in the timed one."""
+    child("""
+for precision in (FP64, FP32_BULK, FP32_MIXED):
+    with gpu.Solver(grid(512, precision=precision)) as s:
+        fake.fake_reset()
+        s.autotune(1)
+        assert fake.fake_most_launches() == 2, precision
+""")
