@@ -13,8 +13,8 @@ floor and thermal-check decisions and the limiter branches are the forward's;
 at a kink the derivative is that of the branch the forward took (one-sided).
 Periodic or outflow sides, each side on its own.
 
-Forward precision: FP64 (the tape kernels, bit-identical to the fused FP64
-step) or a reduced form -- ``FP32_BULK`` or ``FP32_MIXED`` -- in which the
+Forward precision: FP64 (the stage kernels of the fused FP64 step, bit for
+bit) or a reduced form -- ``FP32_BULK`` or ``FP32_MIXED`` -- in which the
 forward steps run through the fused FP32 solver with the same frozen time
 steps (``chimera_set_dt_device`` before each step) and the loss is the
 reduced-precision result.  The checkpoints are that forward's states (as FP64);

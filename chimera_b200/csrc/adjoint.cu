@@ -137,7 +137,7 @@ __device__ __forceinline__ FaceIdx face_idx(const AdjGeom& g, int i, int j, bool
 // Outflow boundary flux correction (src/main.f90:118-148): a cell on an
 // outflow low side gets dt*dx times the physical flux of its own stage
 // primitives, in x (sx) and / or in y (sy).  Same operations as the fused
-// stage kernel's; R = double in the tape, dual numbers in the reverse sweep.
+// stage kernel's, here on dual numbers.
 template <typename R>
 __device__ __forceinline__ void outflow_correction(bool sx, bool sy, R ax, R ay, R gamma, R cr, R cu, R cv, R cP,
                                                    R cBx, R cBy, R* U) {

@@ -1,14 +1,13 @@
 // dual.cuh -- forward-mode dual numbers for the adjoint's local Jacobians.
 //
-// Dual<N> carries a value and N tangents.  Evaluating one of the templated
-// device functions of mhd_device.cuh (get_primitive, the Riemann solvers,
-// conserved_floors, limit_slope) with Dual arguments returns the outputs and
-// their exact derivatives with respect to the seeded inputs, through the same
-// operations and the same branch decisions as the FP64 forward: comparisons
-// look at values only, so at a kink the derivative is that of the branch the
-// forward took (a one-sided derivative), except at an exact tie of a min / max
-// (and |x| at 0), where it is the mean of the two one-sided derivatives.
-// sign() / copysign() have zero derivative in their sign argument.
+// Dual<N> carries a value and N tangents.  Evaluating conserved_floors
+// (mhd_device.cuh) or the outflow correction (adjoint.cu) -- what a few cells only
+// go through, the rest being transposed by hand (face_vjp.cuh) -- with Dual
+// arguments returns the outputs and their exact derivatives with respect to the
+// seeded inputs, through the same operations and the same branch decisions as the
+// FP64 forward: comparisons look at values only, so at a kink the derivative is that
+// of the branch the forward took (a one-sided derivative), except at an exact tie of
+// a maximum, where it is the mean of the two one-sided derivatives.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -52,39 +51,18 @@ template <int N> __device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, 
   return r;
 }
 
-template <int N> __device__ __forceinline__ Dual<N> operator-(const Dual<N>& a) {
+// a plain constant in front (the floors)
+template <int N> __device__ __forceinline__ Dual<N> operator*(double a, const Dual<N>& b) {
   Dual<N> r;
-  r.v = -a.v;
+  r.v = b.v * a;
 #pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = -a.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = b.d[k] * a;
   return r;
 }
-
-// mixed forms with plain doubles
-template <int N> __device__ __forceinline__ Dual<N> operator+(const Dual<N>& a, double b) { return a + Dual<N>(b); }
-template <int N> __device__ __forceinline__ Dual<N> operator+(double a, const Dual<N>& b) { return Dual<N>(a) + b; }
-template <int N> __device__ __forceinline__ Dual<N> operator-(const Dual<N>& a, double b) { return a - Dual<N>(b); }
-template <int N> __device__ __forceinline__ Dual<N> operator-(double a, const Dual<N>& b) { return Dual<N>(a) - b; }
-template <int N> __device__ __forceinline__ Dual<N> operator*(const Dual<N>& a, double b) {
-  Dual<N> r;
-  r.v = a.v * b;
-#pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * b;
-  return r;
-}
-template <int N> __device__ __forceinline__ Dual<N> operator*(double a, const Dual<N>& b) { return b * a; }
-template <int N> __device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, double b) { return a / Dual<N>(b); }
 template <int N> __device__ __forceinline__ Dual<N> operator/(double a, const Dual<N>& b) { return Dual<N>(a) / b; }
 
-#define DUAL_CMP(OP)                                                                                     \
-  template <int N> __device__ __forceinline__ bool operator OP(const Dual<N>& a, const Dual<N>& b) { return a.v OP b.v; } \
-  template <int N> __device__ __forceinline__ bool operator OP(const Dual<N>& a, double b) { return a.v OP b; }            \
-  template <int N> __device__ __forceinline__ bool operator OP(double a, const Dual<N>& b) { return a OP b.v; }
-DUAL_CMP(<)
-DUAL_CMP(>)
-DUAL_CMP(<=)
-DUAL_CMP(>=)
-#undef DUAL_CMP
+template <int N> __device__ __forceinline__ bool operator<(const Dual<N>& a, const Dual<N>& b) { return a.v < b.v; }
+template <int N> __device__ __forceinline__ bool operator>(const Dual<N>& a, const Dual<N>& b) { return a.v > b.v; }
 
 template <int N> __device__ __forceinline__ Dual<N> dsqrt(const Dual<N>& a) {
   Dual<N> r;
@@ -95,47 +73,20 @@ template <int N> __device__ __forceinline__ Dual<N> dsqrt(const Dual<N>& a) {
   return r;
 }
 
-template <int N> __device__ __forceinline__ Dual<N> dcopysign(const Dual<N>& a, const Dual<N>& b) {
-  // |a| with the sign of b; the derivative follows a's magnitude only
-  const bool flip = (signbit(a.v) != signbit(b.v));
-  return flip ? -a : a;
-}
-
-template <int N> __device__ __forceinline__ bool disfinite(const Dual<N>& a) { return isfinite(a.v); }
-
-// min / max of two duals.  At an exact tie -- common here: in a uniform region
-// the left and right face states are bit-identical, so e.g. HLLE's
-// min(vx_L - cf_L, vx_R - cf_R) ties -- the derivative is the mean of the two
-// one-sided ones, which is what a central difference sees; off a tie it is
-// the derivative of the larger / smaller argument.
-template <int N> __device__ __forceinline__ Dual<N> tie_mean(const Dual<N>& a, const Dual<N>& b) {
-  Dual<N> r;
-  r.v = a.v;
+// max of two duals: at an exact tie the derivative is the mean of the two one-sided
+// ones, which is what a central difference sees; off a tie it is that of the larger
+template <int N> __device__ __forceinline__ Dual<N> dmax(const Dual<N>& a, const Dual<N>& b) {
+  if (a.v > b.v) return a;
+  if (b.v > a.v) return b;
+  Dual<N> r(a.v);
 #pragma unroll
   for (int k = 0; k < N; ++k) r.d[k] = 0.5 * (a.d[k] + b.d[k]);
   return r;
 }
-template <int N> __device__ __forceinline__ Dual<N> dmax(const Dual<N>& a, const Dual<N>& b) {
-  return (a.v > b.v) ? a : ((b.v > a.v) ? b : tie_mean(a, b));
-}
-template <int N> __device__ __forceinline__ Dual<N> dmin(const Dual<N>& a, const Dual<N>& b) {
-  return (a.v < b.v) ? a : ((b.v < a.v) ? b : tie_mean(a, b));
-}
-// |x| with zero derivative at x = 0 (the central difference there)
-template <int N> __device__ __forceinline__ Dual<N> dabs(const Dual<N>& a) {
-  return (a.v < 0.0) ? -a : ((a.v > 0.0) ? a : Dual<N>(0.0));
-}
-
-// min / max against plain constants (the floors of mhd_device.cuh)
-template <int N> __device__ __forceinline__ Dual<N> dmax(const Dual<N>& a, double b) { return (a.v > b) ? a : Dual<N>(b); }
-template <int N> __device__ __forceinline__ Dual<N> dmax(double a, const Dual<N>& b) { return (a > b.v) ? Dual<N>(a) : b; }
-template <int N> __device__ __forceinline__ Dual<N> dmin(const Dual<N>& a, double b) { return (a.v < b) ? a : Dual<N>(b); }
-template <int N> __device__ __forceinline__ Dual<N> dmin(double a, const Dual<N>& b) { return (a < b.v) ? Dual<N>(a) : b; }
 
 template <int N> struct K<Dual<N>> {
   static constexpr double P_floor = 1.0e-12;
   static constexpr double rho_floor = 1.0e-12;
-  static constexpr double e_floor_frac = 1.0e-10;
 };
 
 }  // namespace chimera

@@ -10,8 +10,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <type_traits>
-
 namespace chimera {
 
 // src/mhd_config.f90:27-43
@@ -43,12 +41,10 @@ template <> __device__ __forceinline__ float dabs<float>(float a) { return fabsf
 // to be nonzero -- since they can differ from it only in the sign of a zero
 // result or with a NaN second operand.  In FP64 only the absolute value (a
 // sign-bit clear) is cheaper than compare-and-select; FP64 min / max keep it
-// (their IEEE forms measured 20% more instructions on sm_100).  Other
-// argument types (the adjoint's dual numbers) keep the rules of dmax / dmin /
-// dabs.
+// (their IEEE forms measured 20% more instructions on sm_100), and so do the
+// adjoint's dual numbers (hmax).
 template <typename A, typename B> __device__ __forceinline__ auto hmax(A a, B b) { return dmax(a, b); }
 template <typename A, typename B> __device__ __forceinline__ auto hmin(A a, B b) { return dmin(a, b); }
-template <typename A> __device__ __forceinline__ A habs(A a) { return dabs(a); }
 __device__ __forceinline__ double habs(double a) { return fabs(a); }
 __device__ __forceinline__ float hmax(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ float hmin(float a, float b) { return fminf(a, b); }
@@ -60,13 +56,9 @@ __device__ __forceinline__ float dcopysign(float a, float b) { return copysignf(
 __device__ __forceinline__ bool disfinite(double a) { return isfinite(a); }
 
 // sqrt(0.5 (q + |q|)) for q > 0 or NaN: there 0.5 (q + |q|) = 0.5 (2 q) = q
-// exactly (both products by powers of two), so plain float / double take
-// sqrt(q); other arithmetic types (the adjoint's dual numbers) keep the
-// reference's expression (src/mhd_flux.f90:277-278, 355-358).
-template <typename R> __device__ __forceinline__ R sqrt_pos_part(R q) {
-  if constexpr (std::is_floating_point<R>::value) return dsqrt(q);
-  else return dsqrt(R(0.5) * (q + habs(q)));
-}
+// exactly (both products by powers of two): the reference's expression
+// (src/mhd_flux.f90:277-278, 355-358) is sqrt(q).
+template <typename R> __device__ __forceinline__ R sqrt_pos_part(R q) { return dsqrt(q); }
 __device__ __forceinline__ bool disfinite(float a) { return isfinite(a); }
 
 // a / b through a reciprocal y = RN(1/b) fixed for the launch (the cell volume,
@@ -161,15 +153,11 @@ __device__ __forceinline__ R limit_slope(R dfL, R dfR) {
   R den = dfL + dfR;
   if (prod <= R(0) || habs(den) < R(1e-12)) return R(0);
   if (LIMITER == LIMITER_VAN_LEER) return (R(2) * prod) / den;
-  // here dfL and dfR are nonzero with one sign and |den| >= 1e-12
-  if constexpr (std::is_floating_point<R>::value) {
-    // The same value with fewer operations: min(2|a|, 2|b|) = 2 min(|a|, |b|)
-    // (a product by 2 is exact), and sign(1, a) * m = copysign(m, a) for the
-    // non-negative m (a product by +-1 is exact).
-    return dcopysign(hmin(R(2) * hmin(habs(dfL), habs(dfR)), R(0.5) * habs(den)), dfL);
-  } else {   // other arithmetic types (the adjoint's dual numbers): the reference's form
-    return dcopysign(R(1), dfL) * hmin(hmin(R(2) * habs(dfL), R(2) * habs(dfR)), R(0.5) * habs(den));
-  }
+  // Here dfL and dfR are nonzero with one sign and |den| >= 1e-12.  The reference's
+  // value with fewer operations: min(2|a|, 2|b|) = 2 min(|a|, |b|) (a product by 2 is
+  // exact), and sign(1, a) * m = copysign(m, a) for the non-negative m (a product by
+  // +-1 is exact).
+  return dcopysign(hmin(R(2) * hmin(habs(dfL), habs(dfR)), R(0.5) * habs(den)), dfL);
 }
 
 // One face's 5 fluxes in (normal, tangential) orientation.
