@@ -442,16 +442,22 @@ static int run_steps(chimera_handle* h, int nsteps) {
 
 static size_t cells_of(const chimera_cfg& c) { return size_t(c.nx) * size_t(c.ny); }
 
-// Whether the six arrays can be moved by a kernel: float64-aligned memory of the
-// handle's device, and no capture under way (the copies wait for the device, which a
-// capture refuses, as it always has).
-static bool movable(chimera_handle* h, const void* const* ptrs, int where) {
-  if (where != CHIMERA_DEVICE) return false;
+// Whether a stream capture under way refuses a call that reads or sets device state for
+// the host: of the handle's stream, or of another one in a mode that forbids waiting
+// (a query is refused where a wait would be, and does not wait).
+static bool capture_refuses(const chimera_handle* h) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return false;
-  }
+  cudaError_t e = cudaStreamIsCapturing(h->stream, &cs);
+  if (e == cudaSuccess && cs == cudaStreamCaptureStatusNone) e = cudaStreamQuery(h->stream);
+  cudaGetLastError();
+  return cs != cudaStreamCaptureStatusNone || (e != cudaSuccess && e != cudaErrorNotReady);
+}
+
+// Whether the six arrays can be moved by a kernel: float64-aligned memory of the
+// handle's device, and no capture in the way (the copies wait for the device, which a
+// capture refuses).
+static bool movable(chimera_handle* h, const void* const* ptrs, int where) {
+  if (where != CHIMERA_DEVICE || capture_refuses(h)) return false;
   for (int q = 0; q < 6; ++q) {
     cudaPointerAttributes a;
     if (reinterpret_cast<uintptr_t>(ptrs[q]) % sizeof(double) != 0 ||
@@ -1089,9 +1095,7 @@ int chimera_step_host(chimera_handle* h, const double* const* in, double* const*
 int chimera_batch_set_time(chimera_handle* h, int m, double t, int output_count) {
   if (!h || m < 0 || m >= h->n || output_count < 1) return CHIMERA_ERR_BAD_ARG;
   DeviceGuard on(h->device);
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  CK(cudaStreamIsCapturing(h->stream, &cs));
-  if (cs != cudaStreamCaptureStatusNone) return CHIMERA_ERR_CUDA;   // dt_valid is the host's: not for a replay
+  if (capture_refuses(h)) return CHIMERA_ERR_CUDA;   // dt_valid is the host's: not for a replay
   set_time_kernel<<<1, 1, 0, h->stream>>>(h->d_ctl + m, t, output_count, (t < h->cfg[m].t_end) ? 1 : 0);
   CK(cudaGetLastError());
   h->dt_valid[m] = false;

@@ -15,6 +15,7 @@ static int n_kernels = 0;
 static struct { char* p; size_t n; int dev; } blocks[MAX_BLOCKS];
 static long long live = 0;                 /* bytes allocated and not freed */
 static long long limit = 1LL << 60;        /* bytes there are */
+static int capturing = 0;
 static const float* elapsed = 0;           /* what the next event pairs measure */
 static int n_elapsed = 0;
 struct CUstream_st { int dev; };
@@ -22,6 +23,7 @@ struct CUevent_st { int dev; };
 
 /* what a test reads and sets */
 long long fake_live_bytes(void) { return live; }
+void fake_capture(int on) { capturing = on; }   /* of a stream that is not the library's, waiting forbidden */
 void fake_memory(long long bytes) { limit = bytes; }
 int fake_launches(const char* part) {      /* launches of kernels whose name holds part */
   int s = 0;
@@ -139,7 +141,8 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned f) {
   return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; return capturing ? cudaErrorStreamCaptureUnsupported : cudaSuccess; }
+cudaError_t cudaStreamQuery(cudaStream_t s) { (void)s; return capturing ? cudaErrorStreamCaptureUnsupported : cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned f) { (void)s; (void)e; (void)f; return cudaSuccess; }
 cudaError_t cudaStreamGetDevice(cudaStream_t s, int* d) { *d = s->dev; return cudaSuccess; }
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, enum cudaStreamCaptureStatus* c) {

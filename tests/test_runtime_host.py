@@ -112,3 +112,24 @@ for precision in (FP64, FP32_BULK, FP32_MIXED):
         s.autotune(1)
         assert fake.fake_most_launches() == 2, precision
 """)
+
+
+def test_capture_of_another_stream_refuses_state_and_time(child):
+    """set_state, get_state and set_time while the thread captures a stream that forbids
+    waiting: refused before anything is launched, and done again afterwards."""
+    child("""
+with gpu.Solver(grid(16)) as s:
+    dev = [C.c_void_p() for _ in range(6)]
+    for d in dev:
+        assert fake.cudaMalloc(C.byref(d), C.c_size_t(16 * 16 * 8)) == 0
+    def calls():
+        return [lib.chimera_batch_set_state(s.handle, 0, *dev, 16, gpu.DEVICE),
+                lib.chimera_batch_get_state(s.handle, 0, *dev, 16, gpu.DEVICE),
+                lib.chimera_batch_set_time(s.handle, 0, 0.5, 2)]
+    fake.fake_reset()
+    fake.fake_capture(1)
+    assert calls() == [-2, -2, -2]
+    assert fake.fake_launches(b"") == 0
+    fake.fake_capture(0)
+    assert calls() == [0, 0, 0]
+""")
