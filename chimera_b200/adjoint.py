@@ -98,7 +98,8 @@ class Adjoint:
         st, dev = self._stream, t.get_device()
         # (the raw handle: a Stream object each call takes 2.5 us, 4% of a 64^2 gradient)
         if torch._C._cuda_getCurrentRawStream(dev) != st.cuda_stream or dev != st.device_index:
-            st.wait_stream(torch.cuda.current_stream(t.device))
+            if not torch.cuda.is_current_stream_capturing():   # (a capture takes no other stream's events)
+                st.wait_stream(torch.cuda.current_stream(t.device))
 
     def forward_step(self, U, dt):
         out = [torch.empty_like(u) for u in U]

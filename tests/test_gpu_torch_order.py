@@ -103,3 +103,20 @@ def test_set_state_does_not_hold_the_host(A):
         s.set_state(V)
         assert not done.query()
         assert all(np.array_equal(a, b) for a, b in zip(s.get_state(), st))
+
+
+def test_adjoint_in_a_relaxed_capture_runs_at_once(A):
+    """A capture that allows waiting: the call is not part of it and takes no event of
+    the captured stream."""
+    cfg, st = P.orszag_tang(32)
+    U = [torch.from_numpy(x).cuda() for x in st]
+    with A.Adjoint(cfg) as adj:
+        want = adj.forward_step(U, 1e-4)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+            other = torch.ones(4, device="cuda") + 1
+            got = adj.forward_step(U, 1e-4)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        graph.replay()
+        assert torch.equal(other, torch.full_like(other, 2.0))
