@@ -105,3 +105,27 @@ def test_large_batch_bitwise(G, oracle, solver, variant):
             ref = oracle.State(st)
             oracle.run(cfg, ref, 2)
             assert all(np.array_equal(x, y) for x, y in zip(s.get_state(member=m), ref.a)), m
+
+
+@pytest.mark.parametrize("solver", [RUSANOV, HLLE, HLLD])
+def test_every_variant_of_a_batch_bitwise(G, oracle, solver):
+    """The kernels for several grids, in every tile variant: a wide periodic member, an odd
+    one with outflow sides and one smaller than most tiles."""
+    grids = []
+    for k, (nx, ny) in enumerate([(NX, NY), (37, 50), (24, 18)]):
+        cfg, st = P.orszag_tang(max(nx, ny), riemann=solver)
+        cfg = cfg.replace(nx=nx, ny=ny, bc=(BC_OUTFLOW,) * 4 if k == 1 else cfg.bc)
+        grids.append((cfg, _rough([np.ascontiguousarray(a[:ny, :nx]) for a in st], 20 + k)))
+    refs = []
+    for cfg, st in grids:
+        refs.append(oracle.State(st))
+        oracle.run(cfg, refs[-1], 3)
+    with G.Solver([c for c, _ in grids]) as s:
+        for v in range(s.variant_count()):
+            s.set_variant(v)
+            for m, (_, st) in enumerate(grids):
+                s.set_state(st, member=m)
+                s.set_time(0.0, member=m)
+            s.step(3)
+            for m, ref in enumerate(refs):
+                assert all(np.array_equal(x, y) for x, y in zip(s.get_state(member=m), ref.a)), (v, m)
